@@ -184,10 +184,13 @@ size_t walker_smem_bytes(const EngineView& v, bool smem_fields, bool features);
 bool fields_fit_in_smem(const EngineView& v, bool features);
 void launch_init(const EngineView& v, const InitArgs& a, int walkers_per_block, cudaStream_t stream);
 void launch_walk(const EngineView& v, const WalkArgs& a, int walkers_per_block, cudaStream_t stream);
-// sweep.cu: the dense sweep; false when the walker does not fit the shared-memory ring.
+// sweep_ahead.cu: the dense sweep; false when it does not serve the engine (pilot statistics, the
+// Nalivaiko mask, or a walker that does not fit in shared memory).
+bool launch_sweep_ahead(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
+// sweep.cu: the dense sweep with pilot statistics or the Nalivaiko mask; false when the walker
+// does not fit the shared-memory ring, or has neither.
 bool launch_sweep_dense(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
-// The split sweep's possible staging depths for this engine (log2 of the draw / J-row ring);
-// empty when the split sweep does not serve it.
+// The staging depths wlg_engine_set_staging_ring accepts for this engine (log2 of the staged draws).
 std::vector<int> split_ring_logs(const EngineView& v);
 bool launch_sweep_csr(const EngineView& v, const WalkArgs& a, int walkers_per_block, cudaStream_t stream);
 // sweep_window.cu: whole epochs of a single-window run of a dense FP64 system of at most 32

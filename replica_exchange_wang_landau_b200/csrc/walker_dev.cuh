@@ -53,16 +53,9 @@ struct HistStats {
     double coverage;
 };
 
-__device__ __forceinline__ HistStats warp_histogram_statistics(const uint64_t* h, const uint8_t* mask, int nbins,
-                                                               uint64_t active_bins, int lane) {
-    uint64_t covered = 0, mn = ~0ULL, total = 0;
-    for (int b = lane; b < nbins; b += 32) {
-        if (!mask[b]) continue;
-        const uint64_t v = h[b];
-        covered += v != 0 ? 1 : 0;
-        mn = v < mn ? v : mn;
-        total += v;
-    }
+// From each lane's sums over its masked bins: how many have visits, the least and the total visits.
+__device__ __forceinline__ HistStats histogram_statistics_of(uint64_t covered, uint64_t mn, uint64_t total,
+                                                             uint64_t active_bins) {
     covered = warp_sum_u64(covered);
     mn = warp_min_u64(mn);
     total = warp_sum_u64(total);
@@ -81,6 +74,19 @@ __device__ __forceinline__ HistStats warp_histogram_statistics(const uint64_t* h
     s.min_over_mean = s.mean > 0.0 ? static_cast<double>(s.minimum) / s.mean : 0.0;
     s.coverage = static_cast<double>(covered) / static_cast<double>(active_bins);
     return s;
+}
+
+__device__ __forceinline__ HistStats warp_histogram_statistics(const uint64_t* h, const uint8_t* mask, int nbins,
+                                                               uint64_t active_bins, int lane) {
+    uint64_t covered = 0, mn = ~0ULL, total = 0;
+    for (int b = lane; b < nbins; b += 32) {
+        if (!mask[b]) continue;
+        const uint64_t v = h[b];
+        covered += v != 0 ? 1 : 0;
+        mn = v < mn ? v : mn;
+        total += v;
+    }
+    return histogram_statistics_of(covered, mn, total, active_bins);
 }
 
 // flat / covered / ready_for_iteration (src/wang_landau.cpp:369-387)
