@@ -521,6 +521,20 @@ void Engine::build_graph() {
     graph_epochs_ = epochs_per_graph;
 }
 
+// Whether epochs run several to a launch.  A recompute after every epoch comes between them.
+bool Engine::fused_epochs() {
+    if (fused_ < 0) {
+        fused_ = recompute_epochs_ != 1 && p_.exchange_interval <= kFusedEpochAttempts &&
+                         ahead_epochs_fit(view_)
+                     ? 1
+                     : 0;
+        if (fused_ && !d_fused_.ptr)
+            d_fused_.allocate(sizeof(FusedSync) + 2 * walkers_ * sizeof(FusedMail) +
+                              2 * walkers_ * static_cast<uint64_t>(view_.max_window_bins) * sizeof(double));
+    }
+    return fused_ != 0;
+}
+
 void Engine::launch_epochs(uint64_t count) {
     if (window_sweep_) {  // every epoch of the chunk in one launch, no graph
         while (count > 0) {
@@ -528,6 +542,15 @@ void Engine::launch_epochs(uint64_t count) {
             launch_sweep_window(view_, e, stream_);
             count -= e;
         }
+        return;
+    }
+    if (fused_epochs()) {
+        FusedEpochs fe;
+        fe.epochs = static_cast<uint32_t>(count);
+        fe.sync = d_fused_.get<FusedSync>();
+        fe.mail = reinterpret_cast<FusedMail*>(fe.sync + 1);
+        fe.mail_log_g = reinterpret_cast<double*>(fe.mail + 2 * walkers_);
+        launch_ahead_epochs(view_, fe, stream_);
         return;
     }
     WalkArgs a{};
@@ -617,9 +640,11 @@ void Engine::run_epochs(uint64_t max_epochs, uint64_t* epochs_run, int32_t* done
     uint64_t budget = max_epochs;
     while (!done_ && budget > 0) {
         // the single-window kernel runs about a million attempts per walker per launch
-        const uint64_t per_launch =
-            window_sweep_ ? std::clamp<uint64_t>((uint64_t{1} << 20) / std::max<uint64_t>(1, p_.exchange_interval), 1, 4096)
-                          : static_cast<uint64_t>(epochs_per_graph);
+        const uint64_t interval = std::max<uint64_t>(1, p_.exchange_interval);
+        uint64_t per_launch = static_cast<uint64_t>(epochs_per_graph);
+        if (window_sweep_) per_launch = std::clamp<uint64_t>((uint64_t{1} << 20) / interval, 1, 4096);
+        // a launch of several epochs: at least the configured number, about 2^18 attempts per walker
+        else if (fused_epochs()) per_launch = std::clamp<uint64_t>((uint64_t{1} << 18) / interval, std::min<uint64_t>(per_launch, 4096), 4096);
         uint64_t chunk = std::min<uint64_t>(budget, per_launch);
         if (checkpointing_) {
             WalkerState st{};
@@ -950,6 +975,7 @@ void Engine::set_staging_ring(int entries) {
     }
     if (rl == view_.split_ring_log) return;
     view_.split_ring_log = rl;
+    fused_ = -1;  // the walker's shared memory has changed
     // the epoch graph holds the kernels' arguments by value: capture it again
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     if (graph_) cudaGraphDestroy(graph_);

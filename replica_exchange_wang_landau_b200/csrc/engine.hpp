@@ -187,6 +187,25 @@ void launch_walk(const EngineView& v, const WalkArgs& a, int walkers_per_block, 
 // sweep_ahead.cu: the dense sweep; false when it does not serve the engine (pilot statistics, the
 // Nalivaiko mask, or a walker that does not fit in shared memory).
 bool launch_sweep_ahead(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
+// Several epochs and their exchanges in one cooperative launch of that sweep.
+struct FusedSync {         // zeroed before each launch
+    uint32_t arrived;      // walkers that have closed an epoch, counted on
+    uint32_t frozen[3], at_limit[3], failed[3];  // per epoch, three in rotation
+    uint32_t pad[6];
+};
+struct alignas(16) FusedMail {  // a walker's configuration at an epoch's close
+    double energy;
+    int32_t bin, slot;
+};
+struct FusedEpochs {
+    uint32_t epochs = 0;   // 0: one epoch without its exchange
+    FusedSync* sync = nullptr;
+    FusedMail* mail = nullptr;     // 2 x walkers
+    double* mail_log_g = nullptr;  // 2 x walkers x max_window_bins
+};
+// Whether all of the engine's walkers can be resident at once (false too when the sweep does not serve it).
+bool ahead_epochs_fit(const EngineView& v);
+void launch_ahead_epochs(const EngineView& v, const FusedEpochs& epochs, cudaStream_t stream);
 // sweep.cu: the dense sweep with pilot statistics or the Nalivaiko mask; false when the walker
 // does not fit the shared-memory ring, or has neither.
 bool launch_sweep_dense(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
@@ -344,6 +363,13 @@ class Engine {
     void print_progress(bool final_line);
     std::vector<WalkerState> download_states();
 
+    // Epochs of at most this many attempts run several to a launch (launch_ahead_epochs): there a
+    // launch per epoch and the exchange's own kernel cost up to half of an epoch, while in longer
+    // epochs they cost nothing and the walkers' wait for one another stays far below its limit.
+    static constexpr uint64_t kFusedEpochAttempts = 1u << 17;
+    bool fused_epochs();
+    int fused_ = -1;  // -1: not asked yet
+    DeviceBuffer d_fused_;
     bool window_sweep_eligible_ = false;
     bool window_sweep_ = false;
     wlg_run_config cfg_{};
