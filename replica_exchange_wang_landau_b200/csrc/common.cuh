@@ -363,6 +363,8 @@ struct EngineView {
     const float* ell_val32;        // FP32 couplings (FP32 runs)
     int32_t ell_width;             // 32, 64, 128 or 256; 0 when not built
     int32_t spins_global;          // the generic sweep and the initialisation read spins from HBM
+    const double* rows64;          // couplings as full rows for the look-ahead sweep (n x ld): J64 / J32, or
+    const float* rows32;           // a copy of a small cutoff system's, zeros included; null: not served
     int32_t split_ring_log;        // split sweep: log2 of its draw / J-row staging ring (4 or 5; 0 = 4)
     Grid grid;
     int32_t walkers;

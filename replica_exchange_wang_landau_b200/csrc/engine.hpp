@@ -84,6 +84,7 @@ struct DeviceSystem {
     DeviceBuffer pos, axes;
     DeviceBuffer J64, J32, J16, Jscale;
     DeviceBuffer csr_ptr, csr_col, csr_val64, csr_val32;
+    DeviceBuffer rows64, rows32;                 // full rows of a small cutoff system (build_full_rows)
     DeviceBuffer ell_col, ell_val64, ell_val32;  // ELLPACK rows for the CSR sweep
     int32_t ell_width = 0;                       // entries per row (0: not built)
     // cell grid of the CSR build: sites sorted by cell, cells at least the cutoff wide
@@ -218,6 +219,8 @@ bool window_sweep_fits(const EngineView& v);
 void launch_sweep_window(const EngineView& v, uint32_t epochs, cudaStream_t stream);
 void launch_ell_fill(int n, int width, const int32_t* ptr, const int32_t* col, const double* val64,
                      const float* val32, int32_t* ell_col, double* ell_val64, float* ell_val32, cudaStream_t stream);
+// physics.cu: a cutoff system's couplings as full rows (n x ld, zeros where the sites are no neighbours).
+void build_full_rows(DeviceSystem& d, int precision, cudaStream_t stream);
 void launch_exchange(const EngineView& v, cudaStream_t stream);
 // precision.cu: drift measurement and resync after an FP64 recompute of all fields.
 void launch_resync(const EngineView& v, const double* rfields, const double* renergy, PrecisionReport* report,
@@ -368,6 +371,13 @@ class Engine {
     // epochs they cost nothing and the walkers' wait for one another stays far below its limit.
     static constexpr uint64_t kFusedEpochAttempts = 1u << 17;
     bool fused_epochs();
+    // Cutoff systems of at most this many sites and at most four walkers per SM run in the look-ahead
+    // sweep on a copy of their couplings as full rows; a row's zeros change no field (a field is
+    // never -0.0).  The CSR sweep is bound by each walker's memory latency and needs about a
+    // thousand walkers to fill the GPU (10^3 sites, cutoff 2.2: 70 M attempts/s with 64 walkers, 281 M
+    // with 256, 1008 M with 1024; full rows: 405 M, 854 M, 938 M; 12^3 sites, cutoff 1.5, 1024
+    // walkers: 1004 M against 757 M); past 2048 sites a row of 16 KB a flip loses that lead.
+    static constexpr uint64_t kFullRowSites = 2048, kFullRowWalkersPerSm = 4;
     int fused_ = -1;  // -1: not asked yet
     DeviceBuffer d_fused_;
     bool window_sweep_eligible_ = false;

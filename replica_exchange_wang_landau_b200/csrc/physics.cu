@@ -465,6 +465,31 @@ static void build_ellpack(DeviceSystem& d, int precision, int32_t zmax, cudaStre
     }
 }
 
+namespace {
+__global__ void full_rows_kernel(int n, int ld, const int32_t* __restrict__ ptr, const int32_t* __restrict__ col,
+                                 const double* __restrict__ val64, const float* __restrict__ val32, double* rows64,
+                                 float* rows32) {
+    const int row = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (row >= n) return;
+    const size_t base = static_cast<size_t>(row) * static_cast<size_t>(ld);
+    for (int e = ptr[row] + static_cast<int>(threadIdx.x & 31); e < ptr[row + 1]; e += 32) {
+        if (rows64) rows64[base + col[e]] = val64[e];
+        if (rows32) rows32[base + col[e]] = val32[e];
+    }
+}
+}  // namespace
+
+void build_full_rows(DeviceSystem& d, int precision, cudaStream_t stream) {
+    DeviceBuffer& rows = precision == WLG_PRECISION_FP32 ? d.rows32 : d.rows64;
+    rows.allocate(d.n * d.ld * (precision == WLG_PRECISION_FP32 ? sizeof(float) : sizeof(double)));
+    check_cuda(cudaMemsetAsync(rows.ptr, 0, rows.bytes, stream), "memset rows");
+    const unsigned blocks = static_cast<unsigned>((d.n + 7) / 8);
+    full_rows_kernel<<<blocks, 256, 0, stream>>>(static_cast<int>(d.n), static_cast<int>(d.ld), d.csr_ptr.get<int32_t>(),
+                                                 d.csr_col.get<int32_t>(), d.csr_val64.get<double>(),
+                                                 d.csr_val32.get<float>(), d.rows64.get<double>(), d.rows32.get<float>());
+    check_cuda(cudaGetLastError(), "full_rows_kernel");
+}
+
 void upload_couplings(const wlg_couplings& j, DeviceSystem& d, int precision, cudaStream_t stream) {
     d.n = j.n;
     d.ld = (j.n + 15) / 16 * 16;

@@ -223,8 +223,8 @@ template <> struct Stored<WLG_PRECISION_BF16> { using T = __nv_bfloat16; };
 
 template <int kPrec>
 __device__ __forceinline__ const typename Stored<kPrec>::T* coupling_rows(const EngineView& v) {
-    if constexpr (kPrec == WLG_PRECISION_FP64) return v.J64;
-    else if constexpr (kPrec == WLG_PRECISION_FP32) return v.J32;
+    if constexpr (kPrec == WLG_PRECISION_FP64) return v.rows64;
+    else if constexpr (kPrec == WLG_PRECISION_FP32) return v.rows32;
     else return v.J16;
 }
 // One coupling and the pair (2c, 2c + 1) of a row in global memory, widened exactly.
@@ -1350,7 +1350,8 @@ struct AheadLaunch {
 };
 AheadLaunch ahead_launch(const EngineView& v) {
     AheadLaunch l;
-    if (v.csr || v.p.collect || v.p.nalivaiko) return l;
+    if (v.p.collect || v.p.nalivaiko) return l;
+    if (v.csr && !v.rows64 && !v.rows32) return l;
     const bool scaled = v.precision == WLG_PRECISION_BF16;
     l.slots = v.split_ring_log == 5 ? kMaxSlots : kMinSlots;
     if (ahead_layout(v.ld, v.max_window_bins, scaled, l.slots).total > 227 * 1024) l.slots = kMinSlots;
