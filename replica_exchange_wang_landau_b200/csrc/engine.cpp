@@ -300,7 +300,7 @@ void Engine::initialise_walkers(const wlg_run_config& c) {
     v.ell_width = sys_.ell_width;
     int sms = 0;
     check_cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
-    if (sys_.csr && !features_ && n <= kFullRowSites && W <= kFullRowWalkersPerSm * static_cast<uint64_t>(sms))
+    if (sys_.csr && !p_.nalivaiko && n <= kFullRowSites && W <= kFullRowWalkersPerSm * static_cast<uint64_t>(sms))
         build_full_rows(sys_, precision_, stream_);
     v.rows64 = sys_.csr ? sys_.rows64.get<double>() : v.J64;
     v.rows32 = sys_.csr ? sys_.rows32.get<float>() : v.J32;

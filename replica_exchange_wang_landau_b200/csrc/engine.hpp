@@ -185,8 +185,8 @@ size_t walker_smem_bytes(const EngineView& v, bool smem_fields, bool features);
 bool fields_fit_in_smem(const EngineView& v, bool features);
 void launch_init(const EngineView& v, const InitArgs& a, int walkers_per_block, cudaStream_t stream);
 void launch_walk(const EngineView& v, const WalkArgs& a, int walkers_per_block, cudaStream_t stream);
-// sweep_ahead.cu: the dense sweep; false when it does not serve the engine (pilot statistics, the
-// Nalivaiko mask, or a walker that does not fit in shared memory).
+// sweep_ahead.cu: the dense sweep; false when it does not serve the engine (the Nalivaiko mask, a
+// cutoff system without full rows, or a walker that does not fit in shared memory).
 bool launch_sweep_ahead(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
 // Several epochs and their exchanges in one cooperative launch of that sweep.
 struct FusedSync {         // zeroed before each launch
@@ -207,8 +207,8 @@ struct FusedEpochs {
 // Whether all of the engine's walkers can be resident at once (false too when the sweep does not serve it).
 bool ahead_epochs_fit(const EngineView& v);
 void launch_ahead_epochs(const EngineView& v, const FusedEpochs& epochs, cudaStream_t stream);
-// sweep.cu: the dense sweep with pilot statistics or the Nalivaiko mask; false when the walker
-// does not fit the shared-memory ring, or has neither.
+// sweep.cu: the dense sweep with the Nalivaiko mask or, where the look-ahead sweep does not fit, pilot
+// statistics; false when the walker does not fit the shared-memory ring, or has neither.
 bool launch_sweep_dense(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
 // The staging depths wlg_engine_set_staging_ring accepts for this engine (log2 of the staged draws).
 std::vector<int> split_ring_logs(const EngineView& v);

@@ -1,5 +1,5 @@
-// sweep.cu — the dense REWL sweep with pilot statistics or the Nalivaiko mask (without them:
-// sweep_ahead.cu): WangLandauWalker::run_attempts / attempt_flip (src/wang_landau.cpp:244-315) for
+// sweep.cu — the dense REWL sweep with the Nalivaiko mask, with or without pilot statistics (without
+// the mask: sweep_ahead.cu): WangLandauWalker::run_attempts / attempt_flip (src/wang_landau.cpp:244-315) for
 // one batch of exchange_interval attempts, then the walker-local flatness / 1/t check of run_rewl
 // (src/parallel.cpp:395-407).
 //

@@ -21,6 +21,10 @@
 //   fields as of the end of block b - 1, then, following the walker's published decisions, the
 //   flips of block b in order, one fma each.  At the walker's last decision of the block it hands
 //   the lanes over.
+// * the books (one warp, only with pilot statistics): follows the entries as well and keeps the squared
+//   displacements, round trips and representatives on an energy and spins of its own (N = 343,
+//   8 x 4 walkers: 1.69 -> 0.33 us per attempt against the ring sweep that kept them in the walker's
+//   warp).
 // * the remaining warps (fields): after a block, apply its accepted flips to all N fields in
 //   shared memory, each field its flips in order, the J rows read coalesced from L2 with eight
 //   rows in flight; they have the whole next block's time for it.
@@ -55,7 +59,7 @@ constexpr uint32_t kPolls = 1u << 24; // bound of every wait (a poll takes about
 constexpr uint32_t kSyncPolls = 1u << 24;  // of the waits across CTAs (a poll and a sleep, about 0.3 us)
 constexpr int kRoleWarps = 5;         // walker, draws, look-ahead, two pairs warps
 constexpr int kMaxFieldWarps = 8;
-constexpr int kMaxRoles = kRoleWarps + kMaxFieldWarps;
+constexpr int kMaxRoles = kRoleWarps + kMaxFieldWarps;  // one more with pilot statistics
 
 // The role of a CTA's warp.  With the SM to itself (kAlone) the walker also gets a scheduler to
 // itself: warps 4, 8 and 12, which the SM would run on the walker's scheduler, stay idle (the
@@ -63,7 +67,7 @@ constexpr int kMaxRoles = kRoleWarps + kMaxFieldWarps;
 template <bool kAlone>
 __device__ __forceinline__ int role_of(int warp) {
     if constexpr (!kAlone) return warp;
-    return warp == 0 ? 0 : (warp & 3) == 0 ? kMaxRoles : warp - (warp >> 2);
+    return warp == 0 ? 0 : (warp & 3) == 0 ? 2 * kMaxRoles : warp - (warp >> 2);
 }
 __host__ __device__ constexpr int warps_for(int roles, bool alone) { return alone ? roles + (roles - 2) / 3 : roles; }
 
@@ -85,10 +89,11 @@ struct alignas(16) BinRecord {  // one bin of the walker's window
 // A block's attempts: what the walker publishes of each, and (1/t stage) what each adds to log g;
 // both at eight bytes per attempt, so that one running address serves them.
 struct alignas(16) Attempts {
-    uint2 entry[32];  // .x
+    uint2 entry[32];  // .x; .y the bin the attempt started from (pilot statistics)
     double add[32];
+    double field[32]; // local field of the attempt's site (pilot statistics)
 };
-constexpr int kAddWords = 64;  // from entry[i].x to add[i], in words
+constexpr int kAddWords = 64, kFieldWords = 128;  // from entry[i].x to add[i] and to field[i], in words
 
 // What an attempt whose site is draw k needs of the draws, ahead of the couplings of its site with the
 // lanes' sites: one record, two 16-byte loads.
@@ -138,6 +143,8 @@ constexpr int kLastAcc = 13;  // attempts made at the last of them
 constexpr int kSettled = 14;  // field warps that have settled an epoch's end, counted on
 constexpr int kSlot = 15;     // configuration slot of the walker
 constexpr int kReloaded = 16; // warps that have reloaded an exchanged configuration, counted on
+constexpr int kBooked = 17;   // blocks entered in the books (pilot statistics)
+constexpr int kBoundary = 18; // block before whose first attempt the batch has ended, 0: none
 constexpr int kWords = 32;
 
 struct SlotLayout {  // one block record
@@ -154,13 +161,14 @@ __host__ __device__ inline SlotLayout slot_layout(bool scaled) {
     L.total = at;
     return L;
 }
-constexpr size_t kIoBytes = 96;  // EpochIo
+constexpr size_t kIoBytes = 112;  // EpochIo
 constexpr size_t kOwnTable = kStep * sizeof(DrawRecord);
 constexpr size_t kNextTable = kStep * sizeof(NextRecord);
 struct AheadLayout {
-    size_t slots, own_pairs, next_pairs, flips, hand, attempts, ctl, state, io, fields, bins, spins, total;
+    size_t slots, own_pairs, next_pairs, flips, hand, attempts, ctl, state, io, fields, bins, spins;
+    size_t sq, ds, book_spins, total;  // pilot statistics
 };
-__host__ __device__ inline AheadLayout ahead_layout(int ld, int mwb, bool scaled, int slots) {
+__host__ __device__ inline AheadLayout ahead_layout(int ld, int mwb, bool scaled, int slots, bool collect) {
     AheadLayout L;
     size_t at = 0;
     L.slots = at; at += static_cast<size_t>(slots) * slot_layout(scaled).total;
@@ -175,6 +183,9 @@ __host__ __device__ inline AheadLayout ahead_layout(int ld, int mwb, bool scaled
     L.fields = at; at += static_cast<size_t>(ld) * 8;
     L.bins = at; at += (static_cast<size_t>(mwb) + 1) * sizeof(BinRecord);
     L.spins = at; at += round16(static_cast<size_t>(ld));
+    L.sq = at; at += collect ? round16(static_cast<size_t>(mwb) * 8) : 0;
+    L.ds = at; at += collect ? round16(static_cast<size_t>(mwb) * 8) : 0;
+    L.book_spins = at; at += collect ? round16(static_cast<size_t>(ld)) : 0;
     L.total = at;
     return L;
 }
@@ -426,7 +437,9 @@ struct EpochIo {
     double energy, factor;
     int32_t stage, bin, status;
     uint32_t active, forced, batch;
-    uint32_t exchanged, pad;
+    uint32_t exchanged;
+    int32_t rt_state;     // pilot statistics: of the books
+    uint64_t trips;
     uint64_t epoch0, offered;
 };
 
@@ -436,7 +449,7 @@ struct EpochIo {
 // attempt loop costs every attempt: 85 -> 107 us per epoch of the 8x8x8 workload.
 __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& a, const FusedEpochs& fe, EpochIo* io,
                                            WalkerState* st_s, BinRecord* bins, uint32_t* word, int w, int wb, int nbins,
-                                           uint32_t epochs, uint32_t field_warps, int lane) {
+                                           uint32_t epochs, uint32_t settlers, int lane) {
     const DeviceParams& P = v.p;
     const bool fused = fe.epochs != 0;
     const uint32_t batch = io->batch;
@@ -447,7 +460,7 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
     uint64_t offered = io->offered;
     const size_t boff = static_cast<size_t>(w) * static_cast<size_t>(v.grid.count) + static_cast<size_t>(wb);
     // the field warps have brought the fields up to date, in shared memory and in HBM
-    if (wait_at_least(word + kSettled, epochs * field_warps, nullptr) != 0 || ld_relaxed(word + kFail) != 0) {
+    if (wait_at_least(word + kSettled, epochs * settlers, nullptr) != 0 || ld_relaxed(word + kFail) != 0) {
         failed = true;
         if (status == 0) status = WLG_ERR_TIMEOUT;
     }
@@ -466,6 +479,11 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
         st.last_accepted = st.attempted - since;
         st.active_count = io->active;
         st.cur_bin = io->bin;
+        if (P.collect) {
+            st.rt_state = io->rt_state;
+            st.round_trips = io->trips;
+            st.rep_pending = 0;
+        }
         if (a.epoch_mode && st.stage == kWangLandau && (st.attempted - st.last_check >= P.check_interval || at_limit)) {
             // the check reads H: fold the visits into it
             uint64_t covered = 0, least = ~0ULL, total = 0;
@@ -501,6 +519,11 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
             st.slot = c.slot;
             reload = !leave;
             exchanged += c.left ? 1u : 0u;
+            if (P.collect) {
+                round_trip_update(st.energy, window_lower(v, wb), window_lower(v, wb + nbins), P.round_trip_margin,
+                                  st.rt_state, st.round_trips);
+                st.rep_pending = leave ? 1 : 0;  // the books refresh the representatives after the reload
+            }
         }
         offered += static_cast<uint64_t>(c.pairs);
         if (leave && w == 0 && lane == 0) {
@@ -531,8 +554,8 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
     return (leave ? kGoLeave : 0u) | (reload ? kGoReload : 0u);
 }
 
-template <int kPrec, bool kPow2, bool kAlone>
-__global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles - 1, kAlone), kAlone ? 1 : 2) sweep_ahead_kernel(const __grid_constant__ EngineView v,
+template <int kPrec, bool kPow2, bool kAlone, bool kCollect>
+__global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles - 1) + (kCollect ? 1 : 0), kAlone), kAlone ? 1 : 2) sweep_ahead_kernel(const __grid_constant__ EngineView v,
                                                                                                         const __grid_constant__ WalkArgs a,
                                                                                                         int slots, int field_warps,
                                                                                                         const __grid_constant__ FusedEpochs fe) {
@@ -551,7 +574,7 @@ __global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles 
 
     const int ld = v.ld;
     const SlotLayout SL = slot_layout(kScaled);
-    const AheadLayout L = ahead_layout(ld, v.max_window_bins, kScaled, slots);
+    const AheadLayout L = ahead_layout(ld, v.max_window_bins, kScaled, slots, kCollect);
     FlipRecord* flips = reinterpret_cast<FlipRecord*>(smem + L.flips);
     HandWords* hand = reinterpret_cast<HandWords*>(smem + L.hand);
     Attempts* attempts = reinterpret_cast<Attempts*>(smem + L.attempts);
@@ -872,12 +895,19 @@ __global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles 
                 }
                 const int me_hi = accepted ? m_hi : 0;
                 const double m_eff = __hiloint2double(me_hi, 0);
+                [[maybe_unused]] const double h_site = h;
                 h = fma(m_eff, need_u ? d1.x : d0.y, need_u ? fc2 : fc1);
                 up ^= accepted ? static_cast<uint32_t>(__double2loint(d1.y)) : 0u;
                 const uint32_t x = static_cast<uint32_t>(me_hi) | (need_u ? kEntValid | kEntUniform : kEntValid);
                 k = need_u ? k2 : k1;
                 m_hi = sign_of(k);
-                st_relaxed(e_p, x);
+                if constexpr (kCollect) {  // the books read the field and the bin left once the entry is there
+                    *reinterpret_cast<volatile double*>(e_p + kFieldWords) = h_site;
+                    st_relaxed(e_p + 1, static_cast<uint32_t>(cur));
+                    st_release(e_p, x);
+                } else {
+                    st_relaxed(e_p, x);
+                }
                 e_p += 2;
                 fc = fma(m_eff, rl, fc);
                 E = accepted ? Ep : E;
@@ -935,12 +965,13 @@ __global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles 
             io->batch = batch;
             if (failed) st_relaxed(word + kFail, 1u);
             if (failed || !fused) st_release(word + kStop, 1u);
-            // the stop entry; a batch that ended with its block's last draw puts it into the next block's
-            st_release(block_done ? &attempts[(b + 1) & 1u].entry[0].x : e_p, kEntValid | kEntStop);
+            // the stop entry; a batch that ended with its block's last draw has no entry left for it (the
+            // next block's may still be cleared by who follows)
+            st_release(block_done ? word + kBoundary : e_p, block_done ? b + 1 : kEntValid | kEntStop);
             const uint32_t go = wait_go(epochs);
             if (go & kGoLeave) break;
             if (go & kGoReload) {
-                reloads += 1u + static_cast<uint32_t>(field_warps);
+                reloads += 1u + static_cast<uint32_t>(field_warps) + (kCollect ? 1u : 0u);
                 failed = wait_at_least(word + kReloaded, reloads, nullptr) != 0;
             }
             if (block_done) failed = failed || wait_at_least(word + kOwnMade, b + 2, nullptr) != 0;
@@ -1010,6 +1041,7 @@ __global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles 
                 const uint32_t need = b - static_cast<uint32_t>(slots) + 1;
                 int r = wait_at_least(word + kAheadIn, need, word + kStop);
                 if (r == 0) r = wait_at_least(word + kWalkerIn, need, word + kStop);
+                if (kCollect && r == 0) r = wait_at_least(word + kBooked, need, word + kStop);
                 if (r == 2 && lane == 0) st_relaxed(word + kFail, 1u);
                 if (r != 0) break;
             } else if (__all_sync(kFull, ld_relaxed(word + kStop) != 0)) {
@@ -1120,7 +1152,10 @@ __global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles 
                 const double pair = next[k].pair[lane];
                 const uint32_t same = next[k].cross;
                 uint32_t x = ld_relaxed(&e_s[done].x);  // one word: the same for every lane
-                for (uint32_t polls = 0; x == 0 && polls < kPolls; ++polls) x = ld_relaxed(&e_s[done].x);
+                for (uint32_t polls = 0; x == 0 && polls < kPolls; ++polls) {
+                    x = ld_relaxed(&e_s[done].x);
+                    if (done == 0 && x == 0 && b != 0 && ld_relaxed(word + kBoundary) == b) x = kEntValid | kEntStop;
+                }
                 f = fma(__hiloint2double(static_cast<int>(x & 0xC0000000u), 0), pair, f);  // m = 0 unless accepted
                 up ^= (x & 0x40000000u) ? same : 0u;
                 stop = (x & kEntStop) != 0;
@@ -1131,6 +1166,16 @@ __global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles 
             }
             __syncwarp();
             const bool last = stop || gave_up;
+            if constexpr (kCollect) {
+                // the books, too, read the entries: the buffer of the block before, which the walker gets back
+                // with the lanes, is cleared when they are through with it
+                if (!last && b > 0) {
+                    if (wait_at_least(word + kBooked, b, nullptr) != 0) st_relaxed(word + kFail, 1u);
+                    attempts[(b + 1) & 1u].entry[lane] = make_uint2(0, 0);
+                    __syncwarp();
+                    __threadfence_block();
+                }
+            }
             if (!last) {  // hand the lanes over
                 volatile HandWords* out = hand + 33 * ((b + 1) & 1u) + lane;
                 const uint64_t tag = static_cast<uint64_t>(b + 1) << 32;
@@ -1141,7 +1186,7 @@ __global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles 
             const uint32_t x = lane < done ? ld_relaxed(&e_s[lane].x) : 0u;
             const uint32_t neg = __ballot_sync(kFull, x & 0x80000000u), uni = __ballot_sync(kFull, x & kEntUniform);
             const uint32_t skip = __ballot_sync(kFull, x & kEntSkip), acc = __ballot_sync(kFull, x & 0x40000000u);
-            e_s[lane] = make_uint2(0, 0);  // the walker writes there only in block b + 2, or in the next epoch
+            if constexpr (!kCollect) e_s[lane] = make_uint2(0, 0);  // the walker writes there only in block b + 2, or in the next epoch
             // the block's flips for the field warps
             const bool mine_flipped = (acc >> lane) & 1u;
             const int at = mine_flipped ? k0 + lane + __popc(uni & below) : 0;
@@ -1185,14 +1230,21 @@ __global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles 
                     int4* to = reinterpret_cast<int4*>(v.spins + static_cast<size_t>(word[kSlot]) * ld);
                     for (int i = lane; i < (ld >> 4); i += 32) to[i] = reinterpret_cast<const int4*>(sp_s)[i];
                 }
+                const uint32_t settlers = static_cast<uint32_t>(field_warps) + (kCollect ? 1u : 0u);
+                if constexpr (kCollect) {
+                    if (wait_at_least(word + kSettled, epochs * settlers, nullptr) != 0) st_relaxed(word + kFail, 1u);
+                    attempts[0].entry[lane] = make_uint2(0, 0);
+                    attempts[1].entry[lane] = make_uint2(0, 0);
+                }
+                st_relaxed(word + kBoundary, 0u);
                 __syncwarp();
                 const uint32_t go = end_epoch(v, a, fe, reinterpret_cast<EpochIo*>(smem + L.io), st_s, bins, word, w, wb,
-                                              nbins, epochs, static_cast<uint32_t>(field_warps), lane);
+                                              nbins, epochs, settlers, lane);
                 if (go & kGoLeave) break;
                 if (go & kGoReload) {
                     load_spins(static_cast<int>(word[kSlot]), lane, 32);
                     settle(kReloaded);
-                    reloads += 1u + static_cast<uint32_t>(field_warps);
+                    reloads += 1u + settlers;
                     // every field warp's part, too, before the first field is read
                     if (wait_at_least(word + kReloaded, reloads, word + kStop) == 2) st_relaxed(word + kFail, 1u);
                 }
@@ -1316,6 +1368,108 @@ __global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles 
                 settle(kReloaded);
             }
         }
+    } else if (kCollect && role == kRoleWarps + field_warps) {
+        // ---- the books: pilot statistics (src/wang_landau.cpp:272-276, 317-342) ----------------
+        // Follows the walker's entries and keeps, in the reference's order, the squared displacements
+        // and sample counts of the bins, the round trips and the representatives, on an energy and
+        // spins of its own, so that none of it is on the walker's chain.
+        double* sq_s = reinterpret_cast<double*>(smem + L.sq);
+        uint64_t* ds_s = reinterpret_cast<uint64_t*>(smem + L.ds);
+        int8_t* spins = reinterpret_cast<int8_t*>(smem + L.book_spins);
+        EpochIo* io = reinterpret_cast<EpochIo*>(smem + L.io);
+        const double lower = window_lower(v, wb), upper = window_lower(v, wb + nbins);
+        double E = st_s->energy;
+        int32_t rt_state = st_s->rt_state;
+        uint64_t trips = st_s->round_trips;
+        const size_t rep0 = static_cast<size_t>(w) * kRepresentatives + (lane < kRepresentatives ? lane : 0);
+        const double target = v.rep_target[rep0];
+        double nearest = lane < kRepresentatives ? v.rep_dist[rep0] : -1.0;
+        auto represent = [&]() {
+            if (!__any_sync(kFull, fabs(E - target) < nearest)) return;
+            warp_update_representatives(v, w, E, spins, lane);
+            nearest = lane < kRepresentatives ? __ldcg(v.rep_dist + rep0) : -1.0;
+        };
+        auto load_book_spins = [&](int slot) {
+            const int4* from = reinterpret_cast<const int4*>(v.spins + static_cast<size_t>(slot) * ld);
+            for (int i = lane; i < (ld >> 4); i += 32) reinterpret_cast<int4*>(spins)[i] = __ldcg(from + i);
+            __syncwarp();
+        };
+        load_book_spins(st_s->slot);
+        for (int i = lane; i < nbins; i += 32) {
+            sq_s[i] = v.sqdisp[boff + i];
+            ds_s[i] = v.dsamples[boff + i];
+        }
+        __syncwarp();
+        if (st_s->rep_pending) represent();  // a replica exchange changed the configuration
+        int s = 0, k = 0;
+        uint32_t epochs = 0;
+        for (uint32_t b = 0;;) {
+            const int32_t* sites = reinterpret_cast<const int32_t*>(slot_of(s) + SL.site);
+            const Attempts* block = attempts + (b & 1u);
+            int e = 0;
+            bool stop = false, gave_up = false;
+            while (k < kStep) {
+                uint32_t x = ld_relaxed(&block->entry[e].x);
+                for (uint32_t polls = 0; x == 0 && polls < kPolls; ++polls) {
+                    x = ld_relaxed(&block->entry[e].x);
+                    if (e == 0 && x == 0 && b != 0 && ld_relaxed(word + kBoundary) == b) x = kEntValid | kEntStop;
+                }
+                __syncwarp();
+                __threadfence_block();
+                gave_up = x == 0;
+                stop = gave_up || (x & kEntStop) != 0;
+                if (stop) break;
+                if (!(x & kEntSkip)) {
+                    const bool accepted = (x & 0x40000000u) != 0;
+                    const int bin = static_cast<int>(ld_relaxed(&block->entry[e].y));
+                    const double field = *reinterpret_cast<const volatile double*>(&block->field[e]);
+                    const double m = __hiloint2double(static_cast<int>(x & 0xC0000000u), 0);
+                    const double displacement = accepted ? m * field : 0.0;
+                    if (lane == 0) {
+                        sq_s[bin] += displacement * displacement;
+                        ++ds_s[bin];
+                        if (accepted) spins[sites[k]] = (x & 0x80000000u) ? -1 : 1;  // m = -2 * old spin
+                    }
+                    __syncwarp();
+                    if (accepted) {
+                        E = fma(m, field, E);
+                        round_trip_update(E, lower, upper, P.round_trip_margin, rt_state, trips);
+                        represent();
+                    }
+                }
+                k += (x & kEntUniform) ? 2 : 1;
+                ++e;
+            }
+            if (!stop) {
+                __syncwarp();
+                if (lane == 0) st_release(word + kBooked, b + 1);
+                ++b;
+                k -= kStep;
+                s = s + 1 == slots ? 0 : s + 1;
+                continue;
+            }
+            if (lane == 0) {
+                if (gave_up) st_relaxed(word + kFail, 1u);
+                io->rt_state = rt_state;
+                io->trips = trips;
+            }
+            settle(kSettled);
+            const uint32_t go = wait_go(++epochs);
+            if (go & kGoLeave) break;
+            if (go & kGoReload) {
+                load_book_spins(static_cast<int>(word[kSlot]));
+                E = st_s->energy;
+                represent();
+                settle(kReloaded);
+            }
+            rt_state = st_s->rt_state;
+            trips = st_s->round_trips;
+        }
+        if (ld_relaxed(word + kFail) == 0)
+            for (int i = lane; i < nbins; i += 32) {
+                v.sqdisp[boff + i] = sq_s[i];
+                v.dsamples[boff + i] = ds_s[i];
+            }
     }
 
     bar_sync(0, static_cast<int>(blockDim.x));  // every role has left
@@ -1323,22 +1477,26 @@ __global__ void __launch_bounds__(32 * warps_for(kAlone ? kMaxRoles : kMaxRoles 
 
 using AheadFn = void (*)(EngineView, WalkArgs, int, int, FusedEpochs);
 
-template <int kPrec, bool kPow2, bool kAlone>
+template <int kPrec, bool kPow2, bool kAlone, bool kCollect>
 AheadFn ahead_fn() {
     static bool configured = false;
     if (!configured) {
-        check_cuda(cudaFuncSetAttribute(reinterpret_cast<const void*>(&sweep_ahead_kernel<kPrec, kPow2, kAlone>),
+        check_cuda(cudaFuncSetAttribute(reinterpret_cast<const void*>(&sweep_ahead_kernel<kPrec, kPow2, kAlone, kCollect>),
                                         cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
                    "cudaFuncSetAttribute");
         configured = true;
     }
-    return &sweep_ahead_kernel<kPrec, kPow2, kAlone>;
+    return &sweep_ahead_kernel<kPrec, kPow2, kAlone, kCollect>;
 }
 
-template <int kPrec>
+template <int kPrec, bool kCollect>
 AheadFn pick_ahead(bool pow2, bool alone) {
-    if (alone) return pow2 ? ahead_fn<kPrec, true, true>() : ahead_fn<kPrec, false, true>();
-    return pow2 ? ahead_fn<kPrec, true, false>() : ahead_fn<kPrec, false, false>();
+    if (alone) return pow2 ? ahead_fn<kPrec, true, true, kCollect>() : ahead_fn<kPrec, false, true, kCollect>();
+    return pow2 ? ahead_fn<kPrec, true, false, kCollect>() : ahead_fn<kPrec, false, false, kCollect>();
+}
+template <int kPrec>
+AheadFn pick_ahead(bool pow2, bool alone, bool collect) {
+    return collect ? pick_ahead<kPrec, true>(pow2, alone) : pick_ahead<kPrec, false>(pow2, alone);
 }
 
 // How the kernel is launched for an engine; fn is null when the sweep does not serve it.
@@ -1350,24 +1508,25 @@ struct AheadLaunch {
 };
 AheadLaunch ahead_launch(const EngineView& v) {
     AheadLaunch l;
-    if (v.p.collect || v.p.nalivaiko) return l;
+    if (v.p.nalivaiko) return l;
+    const bool collect = v.p.collect != 0;
     if (v.csr && !v.rows64 && !v.rows32) return l;
     const bool scaled = v.precision == WLG_PRECISION_BF16;
     l.slots = v.split_ring_log == 5 ? kMaxSlots : kMinSlots;
-    if (ahead_layout(v.ld, v.max_window_bins, scaled, l.slots).total > 227 * 1024) l.slots = kMinSlots;
-    l.bytes = ahead_layout(v.ld, v.max_window_bins, scaled, l.slots).total;
+    if (ahead_layout(v.ld, v.max_window_bins, scaled, l.slots, collect).total > 227 * 1024) l.slots = kMinSlots;
+    l.bytes = ahead_layout(v.ld, v.max_window_bins, scaled, l.slots, collect).total;
     if (l.bytes > 227 * 1024) return l;
     int device = 0;
     check_cuda(cudaGetDevice(&device), "cudaGetDevice");
     check_cuda(cudaDeviceGetAttribute(&l.sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
     // with more walkers than SMs two CTAs share an SM and its registers
     const bool pow2 = v.grid.pow2_width != 0, alone = v.walkers <= l.sms;
-    l.fn = v.precision == WLG_PRECISION_FP32   ? pick_ahead<WLG_PRECISION_FP32>(pow2, alone)
-           : v.precision == WLG_PRECISION_BF16 ? pick_ahead<WLG_PRECISION_BF16>(pow2, alone)
-                                               : pick_ahead<WLG_PRECISION_FP64>(pow2, alone);
+    l.fn = v.precision == WLG_PRECISION_FP32   ? pick_ahead<WLG_PRECISION_FP32>(pow2, alone, collect)
+           : v.precision == WLG_PRECISION_BF16 ? pick_ahead<WLG_PRECISION_BF16>(pow2, alone, collect)
+                                               : pick_ahead<WLG_PRECISION_FP64>(pow2, alone, collect);
     // one thread per pair of fields, up to eight warps
     l.field_warps = std::max(1, std::min(alone ? kMaxFieldWarps : kMaxFieldWarps - 1, (v.ld / 2 + 31) / 32));
-    l.threads = static_cast<unsigned>(32 * warps_for(kRoleWarps + l.field_warps, alone));
+    l.threads = static_cast<unsigned>(32 * warps_for(kRoleWarps + l.field_warps + (collect ? 1 : 0), alone));
     return l;
 }
 
