@@ -13,6 +13,7 @@
 #include <fstream>
 #include <iostream>
 #include <limits>
+#include <memory>
 #include <mutex>
 #include <sstream>
 
@@ -485,6 +486,10 @@ void Engine::check_device_error() {
     Control ctl{};
     check_cuda(cudaMemcpyAsync(&ctl, d_ctl_.ptr, sizeof ctl, cudaMemcpyDeviceToHost, stream_), "copy control");
     check_cuda(cudaStreamSynchronize(stream_), "epoch");
+    take_control(ctl);
+}
+
+void Engine::take_control(const Control& ctl) {
     done_ = ctl.done != 0;
     epochs_ = ctl.epoch;
     if (ctl.error == WLG_ERR_ESCAPED) throw WlgError(WLG_ERR_ESCAPED, "Walker escaped its energy window");
@@ -496,11 +501,16 @@ void Engine::check_device_error() {
 
 void Engine::inject_wait_timeout() {
     view_.p.withhold_draws = 1;
-    // the epoch graph holds the kernels' arguments by value: capture it again
+    drop_graph();
+}
+
+// The epoch graph holds the kernels' arguments by value: after a change it is captured again.
+void Engine::drop_graph() {
     if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
     if (graph_) cudaGraphDestroy(graph_);
     graph_exec_ = nullptr;
     graph_ = nullptr;
+    primed_ = false;
 }
 
 void Engine::build_graph() {
@@ -511,7 +521,8 @@ void Engine::build_graph() {
     a.fixed_batch = 0;
     a.epoch_mode = 1;
     a.smem_per_walker = static_cast<int32_t>(walker_smem_bytes(view_, smem_fields_, features_));
-    // make sure the kernel attributes are set before capture
+    // make sure the kernel attributes are set and the kernels loaded before capture
+    load_exchange();
     check_cuda(cudaStreamSynchronize(stream_), "sync");
     check_cuda(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal), "begin capture");
     try {
@@ -650,7 +661,9 @@ void Engine::run_epochs(uint64_t max_epochs, uint64_t* epochs_run, int32_t* done
         uint64_t per_launch = static_cast<uint64_t>(epochs_per_graph);
         if (window_sweep_) per_launch = std::clamp<uint64_t>((uint64_t{1} << 20) / interval, 1, 4096);
         // a launch of several epochs: at least the configured number, about 2^18 attempts per walker
-        else if (fused_epochs()) per_launch = std::clamp<uint64_t>((uint64_t{1} << 18) / interval, std::min<uint64_t>(per_launch, 4096), 4096);
+        // (the host looks at checkpoints of all walkers and the progress line between launches, as often as asked)
+        else if (!checkpointing_all_ && cfg_.progress_interval_seconds <= 0.0 && fused_epochs())
+            per_launch = std::max(per_launch, std::min<uint64_t>((uint64_t{1} << 18) / interval, 4096));
         uint64_t chunk = std::min<uint64_t>(budget, per_launch);
         if (checkpointing_) {
             WalkerState st{};
@@ -663,6 +676,7 @@ void Engine::run_epochs(uint64_t max_epochs, uint64_t* epochs_run, int32_t* done
         }
         if (recompute_epochs_ > 1) chunk = std::min(chunk, std::max<uint64_t>(1, next_recompute_ - epochs_));
         launch_epochs(chunk);
+        if (!window_sweep_ && epochs_per_graph > 1 && chunk >= static_cast<uint64_t>(epochs_per_graph)) primed_ = true;
         budget -= std::min(budget, chunk);
         after_epochs();
     }
@@ -717,6 +731,10 @@ void Engine::precision_report(wlg_precision_report* out) {
 // and the progress line.
 void Engine::after_epochs() {
     check_device_error();
+    between_launches();
+}
+
+void Engine::between_launches() {
     if (recompute_epochs_ > 1 && !done_ && epochs_ >= next_recompute_) {
         recompute_fields();
         next_recompute_ = epochs_ + recompute_epochs_;
@@ -734,7 +752,7 @@ void Engine::finish() {
 }
 
 cudaGraph_t Engine::epoch_graph() {
-    if (!graph_exec_) {
+    if (!graph_exec_ && !primed_) {
         WalkArgs a{};
         a.first = 0;
         a.count = static_cast<int32_t>(walkers_);
@@ -742,13 +760,14 @@ cudaGraph_t Engine::epoch_graph() {
         a.smem_per_walker = static_cast<int32_t>(walker_smem_bytes(view_, smem_fields_, features_));
         launch_epoch(a);  // sets the kernel attributes
         after_epochs();
-        build_graph();
     }
+    build_graph();
     return graph_;
 }
 
-void Engine::after_external_epochs() {
-    after_epochs();
+void Engine::after_external_epochs(const Control& ctl) {
+    take_control(ctl);
+    between_launches();
     if (done_) finish();
 }
 
@@ -764,6 +783,7 @@ Batch::Batch(const std::vector<Engine*>& engines) : engines_(engines) {
             if (engines_[j] == engines_[i]) throw WlgError(WLG_ERR_INVALID_ARGUMENT, "an engine appears twice");
     }
     check_cuda(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking), "cudaStreamCreate");
+    check_cuda(cudaMallocHost(&control_, engines_.size() * sizeof(Control)), "cudaMallocHost");
     check_cuda(cudaGraphCreate(&graph_, 0), "cudaGraphCreate");
     for (Engine* e : engines_) {
         cudaGraphNode_t node = nullptr;
@@ -775,6 +795,7 @@ Batch::Batch(const std::vector<Engine*>& engines) : engines_(engines) {
 
 Batch::~Batch() {
     if (stream_) cudaStreamSynchronize(stream_);
+    if (control_) cudaFreeHost(control_);
     if (exec_) cudaGraphExecDestroy(exec_);
     if (graph_) cudaGraphDestroy(graph_);
     if (stream_) cudaStreamDestroy(stream_);
@@ -789,9 +810,13 @@ void Batch::run_epochs(uint64_t max_epochs, uint64_t* launches, int32_t* all_don
     };
     while (budget > 0 && !everyone_done()) {
         check_cuda(cudaGraphLaunch(exec_, stream_), "graph launch");
+        // (read by each engine in turn, 12 us an engine: 1 ms of 96 engines' 8)
+        for (size_t i = 0; i < engines_.size(); ++i)
+            check_cuda(cudaMemcpyAsync(control_ + i, engines_[i]->view().ctl, sizeof(Control), cudaMemcpyDeviceToHost, stream_),
+                       "copy control");
         check_cuda(cudaStreamSynchronize(stream_), "batch");
         ++n;
-        for (Engine* e : engines_) e->after_external_epochs();
+        for (size_t i = 0; i < engines_.size(); ++i) engines_[i]->after_external_epochs(control_[i]);
         budget -= std::min(budget, epochs_per_launch_);
     }
     if (launches) *launches = n;
@@ -885,17 +910,9 @@ void Engine::set_launch(int wpb, int epg) {
     if (wpb) walkers_per_block = wpb;
     if (epg && epg != epochs_per_graph) {
         epochs_per_graph = epg;
-        if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
-        if (graph_) cudaGraphDestroy(graph_);
-        graph_exec_ = nullptr;
-        graph_ = nullptr;
+        drop_graph();
     }
-    if (wpb && graph_exec_) {
-        cudaGraphExecDestroy(graph_exec_);
-        cudaGraphDestroy(graph_);
-        graph_exec_ = nullptr;
-        graph_ = nullptr;
-    }
+    if (wpb) drop_graph();
 }
 
 // Launch-shape autotuner: each candidate (staging ring of the split sweep, walkers per CTA of
@@ -982,11 +999,7 @@ void Engine::set_staging_ring(int entries) {
     if (rl == view_.split_ring_log) return;
     view_.split_ring_log = rl;
     fused_ = -1;  // the walker's shared memory has changed
-    // the epoch graph holds the kernels' arguments by value: capture it again
-    if (graph_exec_) cudaGraphExecDestroy(graph_exec_);
-    if (graph_) cudaGraphDestroy(graph_);
-    graph_exec_ = nullptr;
-    graph_ = nullptr;
+    drop_graph();
 }
 
 int Engine::staging_ring() const {
@@ -1028,14 +1041,27 @@ void Engine::fragment(uint64_t w, int allow_empty, double* log_g, uint64_t* hist
     uint8_t* d_v = reinterpret_cast<uint8_t*>(base + 24 * B);
     int* d_status = reinterpret_cast<int*>(base + ((25 * B + 15) / 16) * 16);
     launch_summarize(view_, static_cast<int>(w), 1, allow_empty, d_lg, d_h, d_se, d_v, d_status, stream_);
-    int status = 0;
-    check_cuda(cudaMemcpyAsync(log_g, d_lg, B * 8, cudaMemcpyDeviceToHost, stream_), "copy");
-    check_cuda(cudaMemcpyAsync(hist, d_h, B * 8, cudaMemcpyDeviceToHost, stream_), "copy");
-    check_cuda(cudaMemcpyAsync(sem, d_se, B * 8, cudaMemcpyDeviceToHost, stream_), "copy");
-    check_cuda(cudaMemcpyAsync(valid, d_v, B, cudaMemcpyDeviceToHost, stream_), "copy");
-    check_cuda(cudaMemcpyAsync(&status, d_status, sizeof status, cudaMemcpyDeviceToHost, stream_), "copy");
+    download_fragments(base, 1, log_g, hist, sem, valid);
+}
+
+// The fragments of `windows` windows, summarized side by side at `base`, in one copy (five copies to
+// pageable memory cost about 10 us each: with the walkers' statistics 130 us of a call on 200 bins,
+// 70 now).
+void Engine::download_fragments(const char* base, size_t windows, double* log_g, uint64_t* hist, double* sem,
+                                uint8_t* valid) {
+    const size_t WB = windows * bins_, status_at = ((25 * WB + 15) / 16) * 16, bytes = status_at + 4 * windows;
+    const std::unique_ptr<char[]> host(new char[bytes]);
+    check_cuda(cudaMemcpyAsync(host.get(), base, bytes, cudaMemcpyDeviceToHost, stream_), "copy");
     check_cuda(cudaStreamSynchronize(stream_), "summarize");
-    if (status) throw WlgError(WLG_ERR_RUNTIME, "Walkers in an energy window have no common active bin");
+    std::memcpy(log_g, host.get(), 8 * WB);
+    std::memcpy(hist, host.get() + 8 * WB, 8 * WB);
+    std::memcpy(sem, host.get() + 16 * WB, 8 * WB);
+    std::memcpy(valid, host.get() + 24 * WB, WB);
+    for (size_t w = 0; w < windows; ++w) {
+        int status = 0;
+        std::memcpy(&status, host.get() + status_at + 4 * w, sizeof status);
+        if (status) throw WlgError(WLG_ERR_RUNTIME, "Walkers in an energy window have no common active bin");
+    }
 }
 
 void Engine::fragments(int allow_empty, double* log_g, uint64_t* hist, double* sem, uint8_t* valid) {
@@ -1049,15 +1075,7 @@ void Engine::fragments(int allow_empty, double* log_g, uint64_t* hist, double* s
     uint8_t* d_v = reinterpret_cast<uint8_t*>(base + 24 * WB);
     int* d_status = reinterpret_cast<int*>(base + status_at);
     launch_summarize(view_, 0, static_cast<int>(windows_), allow_empty, d_lg, d_h, d_se, d_v, d_status, stream_);
-    std::vector<int> status(windows_, 0);
-    check_cuda(cudaMemcpyAsync(log_g, d_lg, WB * 8, cudaMemcpyDeviceToHost, stream_), "copy");
-    check_cuda(cudaMemcpyAsync(hist, d_h, WB * 8, cudaMemcpyDeviceToHost, stream_), "copy");
-    check_cuda(cudaMemcpyAsync(sem, d_se, WB * 8, cudaMemcpyDeviceToHost, stream_), "copy");
-    check_cuda(cudaMemcpyAsync(valid, d_v, WB, cudaMemcpyDeviceToHost, stream_), "copy");
-    check_cuda(cudaMemcpyAsync(status.data(), d_status, 4 * windows_, cudaMemcpyDeviceToHost, stream_), "copy");
-    check_cuda(cudaStreamSynchronize(stream_), "summarize");
-    for (int st : status)
-        if (st) throw WlgError(WLG_ERR_RUNTIME, "Walkers in an energy window have no common active bin");
+    download_fragments(base, windows_, log_g, hist, sem, valid);
 }
 
 void Engine::stitch(int complete_range, double* log_g, uint64_t* hist, double* sem, uint8_t* valid,

@@ -221,6 +221,7 @@ void launch_ell_fill(int n, int width, const int32_t* ptr, const int32_t* col, c
                      const float* val32, int32_t* ell_col, double* ell_val64, float* ell_val32, cudaStream_t stream);
 // physics.cu: a cutoff system's couplings as full rows (n x ld, zeros where the sites are no neighbours).
 void build_full_rows(DeviceSystem& d, int precision, cudaStream_t stream);
+void load_exchange();  // loads the kernel (a stream capture should not)
 void launch_exchange(const EngineView& v, cudaStream_t stream);
 // precision.cu: drift measurement and resync after an FP64 recompute of all fields.
 void launch_resync(const EngineView& v, const double* rfields, const double* renergy, PrecisionReport* report,
@@ -273,6 +274,7 @@ class Batch {
 
   private:
     std::vector<Engine*> engines_;
+    Control* control_ = nullptr;       // pinned, one per engine
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
     cudaStream_t stream_ = nullptr;
@@ -336,7 +338,8 @@ class Engine {
     // batch support: the captured epoch graph (built on first use, after one direct epoch that
     // primes the kernels) and the host work after epochs that a batch launch ran
     cudaGraph_t epoch_graph();
-    void after_external_epochs();
+    const EngineView& view() const { return view_; }
+    void after_external_epochs(const Control& ctl);
     bool is_done() const { return done_; }
     uint64_t epoch_count() const { return epochs_; }
 
@@ -354,9 +357,13 @@ class Engine {
     void configure(const wlg_run_config& c);
     void check_backend(bool csr) const;
     void initialise_walkers(const wlg_run_config& c);
+    void take_control(const Control& ctl);
+    void between_launches();
+    void download_fragments(const char* base, size_t windows, double* log_g, uint64_t* hist, double* sem, uint8_t* valid);
     void check_device_error();
     void launch_epochs(uint64_t count);
     void build_graph();
+    void drop_graph();
     void maybe_checkpoint();
     void recompute_fields();
     void launch_recompute();
@@ -393,6 +400,9 @@ class Engine {
     int precision_ = WLG_PRECISION_FP64;
     cudaStream_t stream_ = nullptr;
     cudaGraphExec_t graph_exec_ = nullptr;
+    // An epoch graph has been built or, where epochs are launched without one, a run of its length has
+    // been made: a batch takes an engine that has neither through one epoch first.
+    bool primed_ = false;
     cudaGraph_t graph_ = nullptr;
     int graph_epochs_ = 0;
 

@@ -316,6 +316,11 @@ __global__ void exchange_pair_kernel(EngineView v, int L, int R, int do_swap, do
 
 // ---- launchers ------------------------------------------------------------------------------
 
+void load_exchange() {
+    cudaFuncAttributes attributes{};
+    check_cuda(cudaFuncGetAttributes(&attributes, exchange_kernel), "cudaFuncGetAttributes");
+}
+
 void launch_exchange(const EngineView& v, cudaStream_t stream) {
     exchange_kernel<<<1, 256, 0, stream>>>(v);
     check_cuda(cudaGetLastError(), "exchange_kernel");

@@ -5,7 +5,7 @@ from __future__ import annotations
 import pytest
 
 from helpers import results_equal, snapshots_equal
-from replica_exchange_wang_landau_b200.engine import Engine, RunConfig, System, run_rewl
+from replica_exchange_wang_landau_b200.engine import Batch, Engine, RunConfig, System, run_rewl
 from replica_exchange_wang_landau_b200.geometry import simple_cubic_random
 
 pytestmark = pytest.mark.gpu
@@ -89,3 +89,20 @@ def test_cutoff_full_rows(oracle, n):
     c.emin, c.emax = -5000.0, 5000.0
     c.resolve_mcs(n)
     assert results_equal(run_rewl(s, c), oracle.run_rewl(s, c)) == []
+
+
+def test_batch_after_epochs():
+    """An engine that has run a graph's worth of epochs enters a batch as it is; one that has not runs one first."""
+    c = _config(0.25, 47, 10_000_000, windows=2, walkers=2, seed=11, overlap=0.75)
+    c.resolve_mcs(33)
+    for before, extra in ((8, 0), (7, 1)):
+        with Engine(_row(33, 4), c) as a, Engine(_row(33, 4), c) as b:
+            a.set_launch(0, 8)
+            a.run_epochs(before)
+            with Batch([a]) as batch:
+                assert a.totals()["epochs"] == before + extra
+                batch.run_epochs(8)
+            b.run_epochs(before + extra + 8)
+            assert a.totals()["epochs"] == b.totals()["epochs"]
+            for w in range(a.walkers):
+                assert snapshots_equal(a.snapshot(w), b.snapshot(w)) == []
