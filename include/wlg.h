@@ -321,8 +321,8 @@ typedef struct wlg_autotune_report {
 } wlg_autotune_report;
 
 /* Launch-shape autotuner: times candidate shapes (walkers per CTA 1-8 for the generic sweep,
- * epochs per graph 4-64, the split sweep's staging depth of 16 or 32 draws with their J rows
- * where both fit in shared memory) on trial_epochs real epochs each through the product path
+ * epochs per graph 4-64 (at least that many to a launch where epochs run many to a launch), the
+ * dense sweep's staging depth of 16 or 32 where it has one) on trial_epochs real epochs each through the product path
  * and keeps the fastest.  The shape never changes results, so the trial epochs count as epochs
  * of the run.  The exchange interval, which changes trajectories, is not tuned.  No
  * counterpart in the reference. */
@@ -331,21 +331,21 @@ wlg_status wlg_engine_autotune(wlg_engine* engine, uint64_t trial_epochs, wlg_au
  * replay (>= 1); 0 leaves a value unchanged.  No counterpart in the reference. */
 wlg_status wlg_engine_set_launch(wlg_engine* engine, int32_t walkers_per_block,
                                  int32_t epochs_per_graph);
-/* The split sweep's staging ring (dense systems up to 1024 sites without pilot statistics or
- * the Nalivaiko mask): entries = 16 or 32 draws, each with its site's J row copied into shared
- * memory ahead of the walker; 0 restores 16.  WLG_ERR_INVALID_ARGUMENT when the engine's sweep
+/* The dense sweep's staging depth (dense systems up to 1024 sites without pilot statistics or
+ * the Nalivaiko mask): entries = 16 (four blocks of 30 draws made ahead of the walker) or 32 (six);
+ * 0 restores 16.  WLG_ERR_INVALID_ARGUMENT when the engine's sweep
  * has no such ring or it does not fit.  Results do not depend on it.  No counterpart in the
  * reference. */
 wlg_status wlg_engine_set_staging_ring(wlg_engine* engine, int32_t entries);
 /* Single-window runs of small dense systems (one window, FP64 couplings, at most 32 sites
- * and 4 walkers, no pilot statistics or Nalivaiko mask) run many epochs per launch in one
- * CTA; this is the default for such engines.  enabled = 0 selects the per-epoch kernels
+ * and 4 walkers, no pilot statistics or Nalivaiko mask) run many epochs per launch, in one
+ * CTA when an epoch has at most 32 attempts; this is the default for such engines.  enabled = 0 selects the per-epoch kernels
  * instead (same results); for other engines the call changes nothing.  No counterpart in
  * the reference. */
 wlg_status wlg_engine_set_window_sweep(wlg_engine* engine, int32_t enabled);
 /* Failure injection, for tests of the bounded device waits (no counterpart in the reference):
- * from the next epoch on, the draw-producer warps of the split sweep (dense systems up to 1024
- * sites) and of the single-window sweep publish no draws, so every walker's wait for its first
+ * from the next epoch on, the draw warps of the look-ahead sweep (dense systems and small
+ * cutoff systems) and of the single-window sweep publish no draws, so every walker's wait for its first
  * draws runs to its limit, the walker records WLG_ERR_TIMEOUT without writing its state back,
  * and the run call returns WLG_ERR_TIMEOUT.  Nothing faults and the device stays usable; the
  * engine itself is finished and should be destroyed.  Other sweeps are not affected. */

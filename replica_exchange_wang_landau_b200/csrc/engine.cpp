@@ -552,8 +552,19 @@ bool Engine::fused_epochs() {
     return fused_ != 0;
 }
 
+// Whether the epochs of a single-window engine run in its own kernel.  That closes an epoch in about 1.3 us
+// within one CTA, and takes 0.23 to 0.32 us per attempt; the look-ahead sweep 4 to 5 us an epoch and 0.117
+// (bin widths that are no power of two: 0.29 and 0.14).  Measured, us per epoch, own kernel / look-ahead sweep:
+// 16 attempts 5.0-6.6 / 6.3-8.4, 32 attempts 8.7-11.9 / 8.1-10.9, 64 attempts 16-23 / 12-16, 1024 attempts
+// 239-342 / 124-158 (8, 27 and 32 sites, 1, 2 and 4 walkers): they meet at 32.
+bool Engine::window_epochs() {
+    if (!window_sweep_) return false;
+    if (ahead_serves_ < 0) ahead_serves_ = ahead_epochs_fit(view_) ? 1 : 0;
+    return p_.exchange_interval <= kWindowEpochAttempts || ahead_serves_ == 0;
+}
+
 void Engine::launch_epochs(uint64_t count) {
-    if (window_sweep_) {  // every epoch of the chunk in one launch, no graph
+    if (window_epochs()) {  // every epoch of the chunk in one launch, no graph
         while (count > 0) {
             const uint32_t e = static_cast<uint32_t>(std::min<uint64_t>(count, 1u << 30));
             launch_sweep_window(view_, e, stream_);
@@ -576,7 +587,7 @@ void Engine::launch_epochs(uint64_t count) {
     a.fixed_batch = 0;
     a.epoch_mode = 1;
     a.smem_per_walker = static_cast<int32_t>(walker_smem_bytes(view_, smem_fields_, features_));
-    if (count == static_cast<uint64_t>(epochs_per_graph) && epochs_per_graph > 1) {
+    if (!window_sweep_ && count == static_cast<uint64_t>(epochs_per_graph) && epochs_per_graph > 1) {
         // first use primes the kernel attributes outside of capture
         if (!graph_exec_) {
             launch_epoch(a);
@@ -656,7 +667,7 @@ void Engine::run_epochs(uint64_t max_epochs, uint64_t* epochs_run, int32_t* done
     const uint64_t start = epochs_;
     uint64_t budget = max_epochs;
     while (!done_ && budget > 0) {
-        // the single-window kernel runs about a million attempts per walker per launch
+        // single-window engines run about a million attempts per walker per launch
         const uint64_t interval = std::max<uint64_t>(1, p_.exchange_interval);
         uint64_t per_launch = static_cast<uint64_t>(epochs_per_graph);
         if (window_sweep_) per_launch = std::clamp<uint64_t>((uint64_t{1} << 20) / interval, 1, 4096);
@@ -703,7 +714,7 @@ void Engine::recompute_fields() {
 // One epoch of run_rewl on the stream: the sweep, the exchange and, when the recompute
 // interval is one epoch, the FP64 recompute.
 void Engine::launch_epoch(const WalkArgs& a) {
-    if (window_sweep_) {
+    if (window_epochs()) {
         launch_sweep_window(view_, 1, stream_);
         return;
     }
@@ -998,7 +1009,7 @@ void Engine::set_staging_ring(int entries) {
     }
     if (rl == view_.split_ring_log) return;
     view_.split_ring_log = rl;
-    fused_ = -1;  // the walker's shared memory has changed
+    fused_ = ahead_serves_ = -1;  // the walker's shared memory has changed
     drop_graph();
 }
 

@@ -376,8 +376,10 @@ class Engine {
     // Epochs of at most this many attempts run several to a launch (launch_ahead_epochs): there a
     // launch per epoch and the exchange's own kernel cost up to half of an epoch, while in longer
     // epochs they cost nothing and the walkers' wait for one another stays far below its limit.
+    static constexpr uint64_t kWindowEpochAttempts = 32;
     static constexpr uint64_t kFusedEpochAttempts = 1u << 17;
     bool fused_epochs();
+    bool window_epochs();
     // Cutoff systems of at most this many sites and at most four walkers per SM run in the look-ahead
     // sweep on a copy of their couplings as full rows; a row's zeros change no field (a field is
     // never -0.0).  The CSR sweep is bound by each walker's memory latency and needs about a
@@ -386,6 +388,7 @@ class Engine {
     // walkers: 1004 M against 757 M); past 2048 sites a row of 16 KB a flip loses that lead.
     static constexpr uint64_t kFullRowSites = 2048, kFullRowWalkersPerSm = 4;
     int fused_ = -1;  // -1: not asked yet
+    int ahead_serves_ = -1;
     DeviceBuffer d_fused_;
     bool window_sweep_eligible_ = false;
     bool window_sweep_ = false;

@@ -653,8 +653,8 @@ class Engine:
 
     @property
     def window_sweep(self) -> bool:
-        """Whether epochs run in the single-window kernel (one window, small dense FP64 system;
-        many epochs per launch).  Setting False selects the per-epoch kernels (same results)."""
+        """Whether the engine is run as a single-window one (one window, small dense FP64 system; many
+        epochs per launch, those of at most 32 attempts in a kernel of their own).  Setting False selects the per-epoch kernels (same results)."""
         return bool(self._lib.wlg_engine_window_sweep(self._h))
 
     @window_sweep.setter

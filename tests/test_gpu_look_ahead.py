@@ -5,7 +5,7 @@ from __future__ import annotations
 import pytest
 
 from helpers import results_equal, snapshots_equal
-from replica_exchange_wang_landau_b200.engine import Batch, Engine, RunConfig, System, run_rewl
+from replica_exchange_wang_landau_b200.engine import Batch, DeviceError, Engine, RunConfig, System, run_rewl
 from replica_exchange_wang_landau_b200.geometry import simple_cubic_random
 
 pytestmark = pytest.mark.gpu
@@ -106,3 +106,32 @@ def test_batch_after_epochs():
             assert a.totals()["epochs"] == b.totals()["epochs"]
             for w in range(a.walkers):
                 assert snapshots_equal(a.snapshot(w), b.snapshot(w)) == []
+
+
+@pytest.mark.parametrize("n", [1, 16, 17, 32])
+@pytest.mark.parametrize("interval", [31, 32, 33, 200000])
+def test_single_window_rule(oracle, n, interval):
+    """Single-window engines on both sides of the interval from which the look-ahead sweep takes their epochs,
+    and beyond the longest epoch that shares a launch."""
+    for width in (0.25, 0.3):
+        c = _config(width, interval, 300000 if interval > 100 else 3000, windows=1, walkers=2, seed=n)
+        c.emin, c.emax = -160 * width, 160 * width
+        c.wl.check_interval_attempts = 10 * interval
+        c.resolve_mcs(n)
+        s = _row(n, n)
+        with Engine(s, c) as e:
+            assert e.window_sweep
+        assert results_equal(run_rewl(s, c), oracle.run_rewl(s, c)) == []
+
+
+@pytest.mark.parametrize("interval", [8, 80])
+def test_single_window_wait_runs_out(interval):
+    c = _config(0.25, interval, 3000, windows=1, walkers=2, seed=3)
+    c.resolve_mcs(8)
+    with Engine(_row(8, 2), c) as e:
+        before = [e.snapshot(w) for w in range(e.walkers)]
+        e.inject_wait_timeout()
+        with pytest.raises(DeviceError) as err:
+            e.run()
+        assert err.value.status == "WLG_ERR_TIMEOUT"
+        assert all(snapshots_equal(e.snapshot(w), before[w]) == [] for w in range(e.walkers))
