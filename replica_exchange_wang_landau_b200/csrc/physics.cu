@@ -288,10 +288,10 @@ __global__ void fields_kernel(EngineView v, const int8_t* __restrict__ spins, in
     const int8_t* s = spins + k * spin_stride;
     double sum = 0.0;
     if (!v.csr) {
-        for (int j = 0; j < v.n; ++j) sum += v.J64[static_cast<size_t>(j) * v.ld + i] * static_cast<double>(s[j]);
+        for (int j = 0; j < v.n; ++j) sum = fma(v.J64[static_cast<size_t>(j) * v.ld + i], static_cast<double>(s[j]), sum);
     } else {
         for (int q = v.csr_ptr[i]; q < v.csr_ptr[i + 1]; ++q)
-            sum += v.csr_val64[q] * static_cast<double>(s[v.csr_col[q]]);
+            sum = fma(v.csr_val64[q], static_cast<double>(s[v.csr_col[q]]), sum);
     }
     fields[k * field_stride + i] = sum;
 }
@@ -299,13 +299,16 @@ __global__ void fields_kernel(EngineView v, const int8_t* __restrict__ spins, in
 // local_fields of dense couplings for G configurations per block.  Each thread owns one site i
 // and keeps G sums; the J column entries J[j][i] are read kFieldPrefetch rows ahead into
 // registers, and the configurations' spins are staged as doubles (+-1.0) in shared memory,
-// TILE rows at a time, so that a term is one multiply and one add, with one shared-memory
+// TILE rows at a time, so that a term is one fma (the product with +-1 is exact, so it rounds as the
+// reference's multiply and add do; as two operations the whole recompute of 256
+// walkers at N = 2458, energies and resync included, took 0.44 ms against 0.37; two sites per thread, which halves
+// the shared-memory broadcasts, changed nothing, 0.37 and 0.38), with one shared-memory
 // broadcast (a double2) per two terms.  Every field is still summed sequentially over j with
-// the reference's operations (sum += J(i, j) * s_j, no contraction), so the result is the one
+// the reference's roundings (sum += J(i, j) * s_j), so the result is the one
 // of fields_kernel whatever G is.  A block reads its sites' columns of J once for G
 // configurations.  G = 8 is used: G = 32 (64 threads, 128 registers) reads J four times less but
 // leaves a quarter of the warps, and the FP64 recompute of 256 walkers at N = 2458 took 0.56 ms
-// with it against 0.43 ms with G = 8.
+// with it against 0.43 ms with G = 8 (both before the fma).
 constexpr int kFieldPrefetch = 8;   // rows of J in flight per thread
 template <int G, int TILE, int THREADS>
 __global__ void __launch_bounds__(THREADS) fields_group_kernel(EngineView v, const int8_t* __restrict__ spins,
@@ -350,8 +353,8 @@ __global__ void __launch_bounds__(THREADS) fields_group_kernel(EngineView v, con
 #pragma unroll
                     for (int g2 = 0; g2 < G / 2; ++g2) {
                         const double2 sg = row[g2];
-                        sum[2 * g2] += jv[u] * sg.x;
-                        sum[2 * g2 + 1] += jv[u] * sg.y;
+                        sum[2 * g2] = fma(jv[u], sg.x, sum[2 * g2]);
+                        sum[2 * g2 + 1] = fma(jv[u], sg.y, sum[2 * g2 + 1]);
                     }
                 }
             }
