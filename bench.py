@@ -63,7 +63,7 @@ def load_peaks() -> dict:
 
 def ncu_traffic_per_launch():
     """dram bytes per sweep-kernel launch from the committed ncu summary, if present."""
-    p = ROOT / "profiles" / "sweep_dense_split_kernel_rewl_n512.md"
+    p = ROOT / "profiles" / "sweep_ahead_kernel_rewl_n512.md"
     if not p.exists():
         return None
     for line in p.read_text().splitlines():
@@ -76,7 +76,7 @@ def ncu_traffic_per_launch():
 
 
 class ClockSampler:
-    """nvidia-smi clocks and throttle reasons sampled every 200 ms during the timed region."""
+    """nvidia-smi clocks and throttle reasons sampled every 20 ms during the timed region."""
 
     FIELDS = ("index,clocks.sm,clocks.max.sm,power.draw,clocks_event_reasons.active,"
               "clocks_event_reasons.hw_slowdown,clocks_event_reasons.hw_thermal_slowdown,"
@@ -85,13 +85,20 @@ class ClockSampler:
     def __init__(self, device: int):
         self.device = device
         self.proc = None
+        self.before = 0  # samples taken before the timed region
         self.file = tempfile.NamedTemporaryFile(mode="w+", suffix=".csv", delete=False)
 
     def __enter__(self):
         try:
             self.proc = subprocess.Popen(
                 ["nvidia-smi", f"--id={self.device}", f"--query-gpu={self.FIELDS}", "--format=csv,noheader,nounits",
-                 "-lms", "200"], stdout=self.file, stderr=subprocess.DEVNULL)
+                 "-lms", "20"], stdout=self.file, stderr=subprocess.DEVNULL)
+            # the timed region is a fraction of a second: start it when the samples have begun to come
+            for _ in range(300):
+                if os.path.getsize(self.file.name) > 0:
+                    break
+                time.sleep(0.01)
+            self.before = len(Path(self.file.name).read_text().splitlines())
         except (FileNotFoundError, OSError):
             self.proc = None
         return self
@@ -114,6 +121,7 @@ class ClockSampler:
                     rows.append(parts)
         finally:
             os.unlink(self.file.name)
+        rows = rows[self.before:] or rows
         if not rows:
             return {"sm_mhz": None, "sm_max_mhz": None, "reasons": ["nvidia-smi unavailable"], "samples": 0}
         sm = [float(r[1]) for r in rows if r[1].replace(".", "").isdigit()]
@@ -176,7 +184,7 @@ def run_ours(args, rank: int, world: int, dist, torch) -> None:
         for _ in range(args.steps):
             flush_l2(torch, flush)
             torch.cuda.synchronize()
-            # the product path: run_epochs (CUDA-graph replays of [sweep, exchange]) with one
+            # the product path: run_epochs (epochs with their exchanges, many to a launch) with one
             # CUDA event before and one after on the engine's stream
             t = eng.time_run(epochs)
             total_ms += t["total_ms"]
@@ -272,7 +280,10 @@ def run_ours(args, rank: int, world: int, dist, torch) -> None:
     # roofline of the sweep kernel: algorithmic bytes = one FP64 J row (N x 8 bytes) per
     # accepted flip (fields, spins and the window's log_g/H live in shared memory)
     peaks = load_peaks()
-    launches = args.steps * epochs
+    # the engine runs at least a graph's epochs and about 2^18 attempts per walker to a launch
+    interval = attempted // (128 * args.steps * epochs)
+    per_launch = max(launch["epochs_per_graph"], min(2 ** 18 // interval, 4096))
+    launches = args.steps * -(-epochs // per_launch)
     k_launches = max(1, kt["epochs"])
     bytes_per_launch = kt["accepted"] * n * 8 / k_launches
     launch_s = (walk_ms / k_launches) / 1e3
@@ -280,7 +291,7 @@ def run_ours(args, rank: int, world: int, dist, torch) -> None:
     traffic = ncu_traffic_per_launch()
 
     cpu = None
-    if rank == 0 and world == 1 and not args.skip_cpu_baseline:
+    if rank == 0 and world == 1 and not args.skip_cpu_baseline and REFERENCE_WL_RUN.exists():
         cpu = cpu_baseline(args.cpu_sample_mcs)
 
     if rank == 0:
@@ -304,7 +315,7 @@ def run_ours(args, rank: int, world: int, dist, torch) -> None:
                             "attempt, differs from the long-running engine of value"},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peaks["hbm_gbs"], "unit": "GB/s",
                          "frac": achieved / peaks["hbm_gbs"], "traffic": traffic,
-                         "kernel": f"sweep_dense_split_kernel<8, pow2 width> (FP64 dense J, "
+                         "kernel": f"sweep_ahead_kernel<FP64, pow2 width> (FP64 dense J, "
                                    f"{launch['staging_ring']}-draw staging ring)", "peak_source": peaks["source"],
                          "bytes_per_launch": bytes_per_launch, "launch_ms": launch_s * 1e3,
                          "acceptance": kt["accepted"] / max(1, kt["attempted"]),
@@ -312,7 +323,7 @@ def run_ours(args, rank: int, world: int, dist, torch) -> None:
                                           f"timed region by a second engine with the same seed, one kernel at a time "
                                           f"with CUDA events around each launch; same attempts and accepted flips "
                                           f"as the timed region (checked)"},
-            "gpu_launches": 2 * launches,
+            "gpu_launches": launches,
             "wall_clock_attempts_per_s": graph_rate,
             "clocks": clock,
             "exchange_ms_per_epoch": exch_ms / k_launches,
