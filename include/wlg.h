@@ -316,7 +316,7 @@ typedef struct wlg_autotune_report {
     int32_t epochs_per_graph;    /* chosen epochs per CUDA-graph replay                        */
     double ms_per_epoch;         /* device time per epoch of the chosen shape                  */
     uint64_t trials;             /* candidate shapes timed                                     */
-    int32_t staging_ring;        /* chosen staging depth of the split sweep (0: not used)      */
+    int32_t staging_ring;        /* chosen staging depth of the dense sweep (0: not used)      */
     int32_t pad;
 } wlg_autotune_report;
 

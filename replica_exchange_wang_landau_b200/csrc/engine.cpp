@@ -926,7 +926,7 @@ void Engine::set_launch(int wpb, int epg) {
     if (wpb) drop_graph();
 }
 
-// Launch-shape autotuner: each candidate (staging ring of the split sweep, walkers per CTA of
+// Launch-shape autotuner: each candidate (staging depth of the dense sweep, walkers per CTA of
 // the generic sweep, epochs per graph replay) runs `trial_epochs` real epochs of this engine
 // through the product path after a warm-up replay that builds its graph, timed with device
 // events; the fastest per epoch is kept.  The candidates are timed twice, in order and then in
@@ -943,7 +943,7 @@ void Engine::autotune(uint64_t trial_epochs, wlg_autotune_report* out) {
     const int* wpbs = generic ? wpbs_generic : wpbs_dense;
     const int n_wpb = generic ? 4 : 1;
     const int epgs[] = {4, 8, 16, 32, 64};
-    // the split sweep's staging depth (16 or 32 draws with their J rows) where it serves the engine
+    // the dense sweep's staging depth where it serves the engine
     std::vector<int> rings;
     for (int rl : split_ring_logs(view_)) rings.push_back(1 << rl);
     if (rings.empty()) rings.push_back(0);

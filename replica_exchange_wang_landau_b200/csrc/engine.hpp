@@ -298,7 +298,7 @@ class Engine {
     void time_run(uint64_t epochs, wlg_epoch_timing* out);
     void autotune(uint64_t trial_epochs, wlg_autotune_report* out);
     void set_launch(int walkers_per_block, int epochs_per_graph);
-    // the split sweep's staging ring (draws with their J rows): 16 or 32 entries, 0 = 16
+    // the dense sweep's staging depth: 16 (four blocks of draws) or 32 (six), 0 = 16
     void set_staging_ring(int entries);
     int staging_ring() const;
     // Failure injection for tests: from the next epoch on, the draw producers of the split and

@@ -13,7 +13,7 @@
 //   value 0 pad a row) with lane j holding entries j, j+32, ...: one coalesced load per
 //   chunk and no row-pointer indirection.
 // * The site of the next attempt is draw hq+1 or, when this attempt consumes the acceptance
-//   uniform, draw hq+2 (the lookahead of the dense split sweep).  The site and both
+//   uniform, draw hq+2 (as in every sweep here).  The site and both
 //   candidates occupy three slots of a four-slot shared-memory ring: each slot receives by
 //   cp.async (no register is the destination of a load in flight, so advancing the ring is
 //   an index change) the site's couplings row, field and spin word, loaded at least one
@@ -34,8 +34,7 @@
 //   and the representative configurations, in the reference's order.
 // * All 32 lanes evaluate the decision chain redundantly; histogram increments go to a
 //   32-bit shared-memory delta per bin that is folded into H at the end of the batch, and the
-//   Wang-Landau count of active bins is updated once from the visited mask, as in the dense
-//   split sweep.
+//   Wang-Landau count of active bins is updated once from the visited mask.
 // The kernel has no waits on other warps or kernels.  Bit-exactness of the rearranged
 // arithmetic is argued where the dense sweeps use the same forms (E + (-2s)h as fma(m, h, E);
 // the power-of-two bin index as fma(E', 1/width, -min/width); the acceptance test

@@ -7,7 +7,8 @@
 // The per-epoch launches of the other sweeps (a kernel node for the walk and one for the
 // exchange, each staging the walker state in and out) cost a few microseconds, which is
 // most of an epoch when a system has a handful of spins and the exchange interval is tens
-// of attempts.  Here one CTA holds every walker of the window for many epochs:
+// of attempts.  Here one CTA holds every walker of the window for many epochs (the engine runs epochs
+// of at most 32 attempts this way, longer ones in the look-ahead sweep: Engine::window_epochs):
 //
 // * Warp w < W is walker w's decision warp, warp W + w its draw producer (W walkers).
 // * N <= 32: lane j keeps the field of site j in a register and the spins are a 32-bit mask
@@ -15,7 +16,7 @@
 //   updates every field at once, f_j = fma(m_eff, J_ij, f_j) on lane j, with m_eff = 0 for a
 //   rejected flip (exact: a field is never -0.0, as the sums start at +0.0).
 // * The next attempt's site is draw hq+1 or, when this attempt consumes the acceptance
-//   uniform, draw hq+2 (the lookahead of the dense split sweep): both candidates' fields are
+//   uniform, draw hq+2: both candidates' fields are
 //   read by shuffles before the decision, and the chosen one is brought up to date with one
 //   fma after it, so the chain is field -> proposed energy -> bin -> log g -> accept ->
 //   next field, with no memory access but the log g load.
@@ -31,7 +32,7 @@
 // * Every wait on another warp is bounded: a walker that waits too long for draws records
 //   WLG_ERR_TIMEOUT, still takes part in the epoch's barrier (so the others end the run at
 //   that epoch) and does not write its state back.
-// The decision arithmetic is that of the split sweep, operation for operation.
+// The decision arithmetic is that of the look-ahead sweep, operation for operation.
 #include <type_traits>
 
 #include "engine.hpp"

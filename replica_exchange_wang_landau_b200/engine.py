@@ -639,11 +639,11 @@ class Engine:
         _check(fn(self._h, _dptr(lg), float(factor)))
 
     def set_staging_ring(self, entries: int) -> None:
-        """The split sweep's staging ring: 16 or 32 draws with their J rows (0 = 16)."""
+        """The dense sweep's staging depth: 16 (four blocks of draws) or 32 (six); 0 = 16."""
         _check(self._lib.wlg_engine_set_staging_ring(self._h, int(entries)))
 
     def inject_wait_timeout(self) -> None:
-        """Failure injection for tests: the draw producers of the split and single-window sweeps
+        """Failure injection for tests: the draw warps of the look-ahead and single-window sweeps
         publish nothing from the next epoch on, so the walkers' bounded waits run out and the
         next run call raises a DeviceError with status WLG_ERR_TIMEOUT."""
         _check(self._lib.wlg_engine_inject_wait_timeout(self._h))
