@@ -373,10 +373,11 @@ class Engine {
     void print_progress(bool final_line);
     std::vector<WalkerState> download_states();
 
+    // Single-window engines' epochs of at most this many attempts run in their own kernel (window_epochs).
+    static constexpr uint64_t kWindowEpochAttempts = 32;
     // Epochs of at most this many attempts run several to a launch (launch_ahead_epochs): there a
     // launch per epoch and the exchange's own kernel cost up to half of an epoch, while in longer
     // epochs they cost nothing and the walkers' wait for one another stays far below its limit.
-    static constexpr uint64_t kWindowEpochAttempts = 32;
     static constexpr uint64_t kFusedEpochAttempts = 1u << 17;
     bool fused_epochs();
     bool window_epochs();
