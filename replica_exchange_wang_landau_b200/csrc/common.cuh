@@ -203,6 +203,18 @@ WLG_HD double floor_near_integer(double offset, double width, double n) {
     return fma(-n, width, offset) >= -half_below * width ? n : n - 1.0;
 }
 
+// ---- the bin an epoch starts from -------------------------------------------------------
+//
+// An exchange may bring a configuration whose bin its new walker has not visited; the next attempt visits
+// it if the walker stays there (update_current_bin, src/wang_landau.cpp:290-303).  `active` counts the
+// visited bins but not that one, `before` are the values ahead of the attempt.  An accepted flip within the
+// bin finds it unvisited and has counted it itself, one to another bin leaves it as it was; so a walker in
+// the same bin with the same count has rejected the flip and has to count its bin.  The walker's own bin and
+// count say so, not the entry it has published of the attempt, which its reader clears.
+WLG_HD bool opened_by_staying(int bin, int bin_before, uint32_t active, uint32_t active_before) {
+    return bin == bin_before && active == active_before;
+}
+
 // ---- the histogram mean of histogram_statistics (src/wang_landau.cpp:349-361) --------
 //
 // The reference sums the histogram in long double (x87, 64-bit significand) and computes

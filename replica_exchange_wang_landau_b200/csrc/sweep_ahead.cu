@@ -437,7 +437,8 @@ __device__ __forceinline__ EpochClose close_epoch(const EngineView& v, const Fus
     return c;
 }
 
-// What the walker leaves for the look-ahead warp's end_epoch, and finds there afterwards.
+// What the walker leaves for the look-ahead warp's end_epoch, and finds there afterwards: in an epoch, bin
+// and active are those of its start.
 struct EpochIo {
     double energy, factor;
     int32_t stage, bin, status;
@@ -658,6 +659,13 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
         uint32_t n_forced = 0;
         uint32_t active32 = static_cast<uint32_t>(ws->active_count);  // at most the window's bins
         int cur = escaped ? 0 : ws->cur_bin - wb;
+        EpochIo* io = reinterpret_cast<EpochIo*>(smem + L.io);
+        static_assert(sizeof(EpochIo) <= kIoBytes, "EpochIo");
+        io->bin = cur + wb;
+        io->active = active32;
+        io->exchanged = 0;
+        io->offered = 0;
+        io->epoch0 = ctl->epoch;
         int s = 0;
         uint32_t k = 0;  // draw (lane) of the current attempt's site
         int status = escaped ? WLG_ERR_ESCAPED : 0;
@@ -749,7 +757,9 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
                         const uint32_t made = static_cast<uint32_t>(e_p - e_mark) >> 1;
                         if (made != 0) {
                             // an initial bin not visited before is opened by the first attempt if that stayed there
-                            if (t == 0 && opens && !(e_mark[0] & 0x40000000u)) ++active32;
+                            // (the epoch's bin and count are where its start left them: the look-ahead warp may
+                            // have cleared the attempt's entry by now, when it was the block's last)
+                            if (t == 0 && opens && opened_by_staying(cur + wb, io->bin, active32, io->active)) ++active32;
                             if (kIT)
                                 factor = __shfl_sync(kFull, quotient, static_cast<int>((e_p - quotient_mark) >> 1) - 1);
                             t += made;
@@ -937,11 +947,6 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
         const bool top_window = wb + nbins == static_cast<int>(g.count);
         // (no branch on the lane number and no call in this loop: see end_epoch)
         uint32_t reloads = 0;  // warps that have to have reloaded
-        EpochIo* io = reinterpret_cast<EpochIo*>(smem + L.io);
-        static_assert(sizeof(EpochIo) <= kIoBytes, "EpochIo");
-        io->exchanged = 0;
-        io->offered = 0;
-        io->epoch0 = ctl->epoch;
         for (uint32_t epochs = 1;; ++epochs) {
             const uint64_t made = st_s->attempted;
             uint64_t left = a.fixed_batch ? a.fixed_batch : P.exchange_interval;
