@@ -138,8 +138,8 @@ constexpr int kWalkerIn = 3;  // block the walker is in
 constexpr int kStop = 4;      // the walker has ended its last batch
 constexpr int kFail = 5;      // a bounded wait gave up
 constexpr int kFinal = 6;     // the flips handed to the field warps are the batch's last
-constexpr int kGo = 1;        // epochs closed: (count << 2) | kGoLeave | kGoReload
-constexpr uint32_t kGoLeave = 1u, kGoReload = 2u;
+constexpr int kGo = 1;        // epochs closed: (count << 2) | flags
+constexpr uint32_t kGoLeave = 1u, kGoReload = 2u, kGoGaveUp = 3u;  // (kGoGaveUp: leave, a role did not get the word)
 constexpr int kCount = 8;     // [8], [9]: flips of the two flip lists
 constexpr int kOwnMade = 10;  // blocks whose own pairs are gathered
 constexpr int kNextMade = 11; // blocks whose pairs with the next block are gathered
@@ -510,7 +510,7 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
             if (stats_ready(hs, st.stage, P)) warp_begin_next_iteration(st, v.hist + boff, nullptr, nbins, P, lane);
         }
     }
-    bool leave = true, reload = false;
+    bool leave = true, reload = false, done = false;
     if (fused) {
         // every walker arrives with its configuration's energy and bin, and each pair's two walkers
         // then decide their exchange alike
@@ -532,13 +532,10 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
             }
         }
         offered += static_cast<uint64_t>(c.pairs);
-        if (leave && w == 0 && lane == 0) {
-            v.ctl->exchange_attempted += offered;
-            v.ctl->epoch = epoch0 + epochs;
-            v.ctl->done = c.done || failed ? 1 : 0;
-        }
+        done = c.done;
     }
     __syncwarp();
+    uint32_t flags = (leave ? kGoLeave : 0u) | (reload ? kGoReload : 0u);
     if (lane == 0) {
         if (failed) {
             st_relaxed(word + kFail, 1u);
@@ -553,11 +550,20 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
         io->status = status;
         io->exchanged = exchanged;
         io->offered = offered;
-        if (leave) st_release(word + kStop, 1u);
-        st_release(word + kGo, (epochs << 2) | (leave ? kGoLeave : 0u) | (reload ? kGoReload : 0u));
+        // The word is replaced, not stored: a role that has given up waiting for it has put its own there,
+        // and then this warp leaves as well (it would otherwise wait at a barrier for warps that have left).
+        __threadfence_block();
+        const uint32_t before = ld_relaxed(word + kGo);
+        if ((before >> 2) == (epochs & 0x3fffffffu) || atomicCAS(word + kGo, before, (epochs << 2) | flags) != before)
+            flags = kGoGaveUp;
+        if (flags & kGoLeave) st_release(word + kStop, 1u);
+        if (fused && w == 0 && (flags & kGoLeave)) {
+            v.ctl->exchange_attempted += offered;
+            v.ctl->epoch = epoch0 + epochs;
+            v.ctl->done = done || failed || flags == kGoGaveUp ? 1 : 0;
+        }
     }
-    __syncwarp();
-    return (leave ? kGoLeave : 0u) | (reload ? kGoReload : 0u);
+    return __shfl_sync(kFull, flags, 0);
 }
 
 template <int kPrec, bool kPow2, bool kAlone, bool kCollect>
@@ -635,18 +641,25 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
             atomicAdd(word + counter, 1u);
         }
     };
-    // Waits for the word on the end of epoch `count`; the flags, or kGoLeave when that never came.
+    // Waits for the word on the end of epoch `count`; its flags.  A role that gives up puts a word of its own in
+    // place of the one it saw last, for all: either the look-ahead warp's word came first and holds, or every
+    // role, the look-ahead warp among them, leaves (by all lanes: no branch on the lane number here).
     auto wait_go = [&](uint32_t count) -> uint32_t {
+        uint32_t x = 0;
         for (uint32_t polls = 0; polls < kSyncPolls; ++polls) {
-            const uint32_t x = ld_relaxed(word + kGo);
+            x = ld_relaxed(word + kGo);
             if (__all_sync(kFull, (x >> 2) == (count & 0x3fffffffu))) {
                 __threadfence_block();
                 return __shfl_sync(kFull, x, 0) & 3u;
             }
             __nanosleep(100);
         }
-        st_relaxed(word + kFail, 1u);
-        return kGoLeave;
+        atomicCAS(word + kGo, x, (count << 2) | kGoGaveUp);
+        __syncwarp();
+        __threadfence_block();
+        x = __shfl_sync(kFull, ld_relaxed(word + kGo), 0) & 3u;
+        if (x == kGoGaveUp) st_relaxed(word + kFail, 1u);
+        return x;
     };
 
     auto slot_of = [&](int s) { return smem + L.slots + static_cast<size_t>(s) * SL.total; };
@@ -1007,7 +1020,8 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
         }
         bar_sync(0, static_cast<int>(blockDim.x));  // every role has left
         if (failed || ld_relaxed(word + kFail) != 0) {
-            if (lane == 0 && !fused) record_error(ctl, io->status > 0 ? io->status : WLG_ERR_TIMEOUT, w);
+            // (in a launch of several epochs the first error is there already, unless a role gave up since)
+            if (lane == 0) record_error(ctl, io->status > 0 ? io->status : WLG_ERR_TIMEOUT, w);
             return;
         }
         const uint32_t exchanged = io->exchanged;

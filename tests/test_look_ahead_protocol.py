@@ -3,7 +3,11 @@ beside it.
 
 The walker publishes an entry per attempt; the look-ahead warp follows the entries of a block and clears
 them once it has read the last one, at a time of its own.  So nothing that the walker decides may depend
-on an entry it has published.  No GPU is involved."""
+on an entry it has published.
+
+At an epoch's end the look-ahead warp publishes one word that says whether the roles go on.  Every wait for it
+is bounded, and a role that goes on meets the others at barriers: so all roles have to take the same word,
+also when one of them gives up waiting while the look-ahead warp is about to publish.  No GPU is involved."""
 from __future__ import annotations
 
 import itertools
@@ -66,3 +70,45 @@ def test_opened_by_staying(tmp_path):
                     str(ROOT / "tests" / "native" / "opened_bin_check.cpp"), "-o", str(exe)], check=True)
     res = subprocess.run([str(exe)], capture_output=True, text=True)
     assert res.returncode == 0 and res.stdout.startswith("ok"), res.stdout
+
+
+def _epoch_end(replaces: bool, waiting: int = 2):
+    """All outcomes of an epoch's end: `waiting` roles that look at the word at any time and give up at any
+    later one, against the look-ahead warp that publishes "go on" at any time.  The word is 0 until then;
+    with `replaces` it is replaced by compare-and-swap, else stored, and a role that gives up just leaves."""
+    seen = set()
+
+    def step(word, roles, ahead):
+        if all(r in ("on", "left") for r in roles) and ahead in ("on", "left"):
+            seen.add(tuple(sorted({*roles, ahead})))
+            return
+        if ahead == "before":
+            if not replaces:
+                step("on", roles, "on")
+            else:
+                step(word or "on", roles, "left" if word == "left" else "on")
+        for i, r in enumerate(roles):
+            if r != "waits":
+                continue
+            to = lambda x: roles[:i] + (x,) + roles[i + 1:]
+            if word:
+                step(word, to("on" if word == "on" else "left"), ahead)
+            elif replaces:  # gives up: its word for all
+                step("left", to("left"), ahead)
+            else:
+                step(word, to("left"), ahead)
+
+    step("", ("waits",) * waiting, "before")
+    return seen
+
+
+def test_all_roles_take_the_same_word_at_an_epochs_end():
+    assert _epoch_end(True) == {("on",), ("left",)}
+    # the model is not vacuous: with a plain store one role leaves and the others wait for it at a barrier
+    assert ("left", "on") in _epoch_end(False)
+
+
+def test_the_word_is_replaced_by_compare_and_swap():
+    body = re.sub(r"//[^\n]*", "", SOURCE)
+    assert len(re.findall(r"atomicCAS\(word \+ kGo,", body)) == 2
+    assert re.findall(r"st_(?:release|relaxed)\(word \+ kGo,", body) == []
