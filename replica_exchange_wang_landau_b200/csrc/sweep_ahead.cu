@@ -150,6 +150,7 @@ constexpr int kSlot = 15;     // configuration slot of the walker
 constexpr int kReloaded = 16; // warps that have reloaded an exchanged configuration, counted on
 constexpr int kBooked = 17;   // blocks entered in the books (pilot statistics)
 constexpr int kBoundary = 18; // block before whose first attempt the batch has ended, 0: none
+constexpr int kEnded = 19;    // epochs the walker has ended (what it leaves in EpochIo is complete)
 constexpr int kWords = 32;
 
 struct SlotLayout {  // one block record
@@ -458,6 +459,11 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
                                            uint32_t epochs, uint32_t settlers, int lane) {
     const DeviceParams& P = v.p;
     const bool fused = fe.epochs != 0;
+    // A look-ahead warp that has given up comes here ahead of the walker, whose own waits then run out, each
+    // within kPolls of its faster polls.
+    int walker_ended = 2;
+    for (int tries = 0; tries < 4 && walker_ended != 0; ++tries)
+        walker_ended = wait_at_least(word + kEnded, epochs, nullptr);
     const uint32_t batch = io->batch;
     const uint64_t epoch0 = io->epoch0;
     int status = io->status;
@@ -466,7 +472,7 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
     uint64_t offered = io->offered;
     const size_t boff = static_cast<size_t>(w) * static_cast<size_t>(v.grid.count) + static_cast<size_t>(wb);
     // the field warps have brought the fields up to date, in shared memory and in HBM
-    if (wait_at_least(word + kSettled, epochs * settlers, nullptr) != 0 || ld_relaxed(word + kFail) != 0) {
+    if (walker_ended != 0 || wait_at_least(word + kSettled, epochs * settlers, nullptr) != 0 || ld_relaxed(word + kFail) != 0) {
         failed = true;
         if (status == 0) status = WLG_ERR_TIMEOUT;
     }
@@ -630,6 +636,14 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
     if (threadIdx.x < 66) hand[threadIdx.x] = HandWords{0, 0};
     if (threadIdx.x < kWords) word[threadIdx.x] = 0;
     if (threadIdx.x == 32) *st_s = *ws;
+    static_assert(sizeof(EpochIo) <= kIoBytes, "EpochIo");
+    if (threadIdx.x == 64) {
+        EpochIo first{};
+        first.bin = escaped ? wb : ws->cur_bin;
+        first.active = static_cast<uint32_t>(ws->active_count);
+        first.epoch0 = ctl->epoch;
+        *reinterpret_cast<EpochIo*>(smem + L.io) = first;
+    }
     __syncthreads();
     if (threadIdx.x == 0) word[kSlot] = static_cast<uint32_t>(st_s->slot);
     __syncthreads();
@@ -673,12 +687,6 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
         uint32_t active32 = static_cast<uint32_t>(ws->active_count);  // at most the window's bins
         int cur = escaped ? 0 : ws->cur_bin - wb;
         EpochIo* io = reinterpret_cast<EpochIo*>(smem + L.io);
-        static_assert(sizeof(EpochIo) <= kIoBytes, "EpochIo");
-        io->bin = cur + wb;
-        io->active = active32;
-        io->exchanged = 0;
-        io->offered = 0;
-        io->epoch0 = ctl->epoch;
         int s = 0;
         uint32_t k = 0;  // draw (lane) of the current attempt's site
         int status = escaped ? WLG_ERR_ESCAPED : 0;
@@ -986,6 +994,7 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
             io->active = active32;
             io->forced = n_forced;
             io->batch = batch;
+            st_release(word + kEnded, epochs);
             if (failed) st_relaxed(word + kFail, 1u);
             if (failed || !fused) st_release(word + kStop, 1u);
             // the stop entry; a batch that ended with its block's last draw has no entry left for it (the

@@ -112,3 +112,16 @@ def test_the_word_is_replaced_by_compare_and_swap():
     body = re.sub(r"//[^\n]*", "", SOURCE)
     assert len(re.findall(r"atomicCAS\(word \+ kGo,", body)) == 2
     assert re.findall(r"st_(?:release|relaxed)\(word \+ kGo,", body) == []
+
+
+def test_the_epochs_end_waits_for_the_walker():
+    """A look-ahead warp that gives up is ahead of the walker: what the walker leaves for the epoch's end is
+    initialised before the roles part, and read after the walker has said that it is complete."""
+    body = SOURCE[SOURCE.index("__noinline__ uint32_t end_epoch("):SOURCE.index("template <int kPrec, bool kPow2, bool kAlone")]
+    ended = body.index("wait_at_least(word + kEnded, epochs, nullptr)")
+    assert ended < min(m.start() for m in re.finditer(r"io->", body))
+    staging = SOURCE[SOURCE.index("// ---- stage the walker"):SOURCE.index("// ---- the walker ---")]
+    assert "EpochIo first{};" in staging
+    walker = SOURCE[SOURCE.index("// ---- the walker ---"):SOURCE.index("// ---- draws ---")]
+    end = walker[walker.index("io->energy = E;"):]
+    assert end.index("io->batch = batch;") < end.index("st_release(word + kEnded, epochs)") < end.index("kEntStop")
