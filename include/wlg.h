@@ -350,6 +350,11 @@ wlg_status wlg_engine_set_window_sweep(wlg_engine* engine, int32_t enabled);
  * and the run call returns WLG_ERR_TIMEOUT.  Nothing faults and the device stays usable; the
  * engine itself is finished and should be destroyed.  Other sweeps are not affected. */
 wlg_status wlg_engine_inject_wait_timeout(wlg_engine* engine);
+/* The same for one walker (-1: all), whose draw warp publishes `blocks` blocks of draws (30 draws in the
+ * look-ahead sweep, 32 in the single-window sweep) of each launch and no more: its wait runs out in the
+ * middle of the launch.  Where epochs share a launch the run ends with the epoch in which that happens:
+ * the other walkers have made it, the failed one has the state it had before it. */
+wlg_status wlg_engine_inject_wait_timeout_at(wlg_engine* engine, int64_t walker, uint32_t blocks);
 /* 1 when the engine runs its epochs with the single-window kernel, else 0. */
 int32_t wlg_engine_window_sweep(const wlg_engine* engine);
 /* The drift report of a mixed-precision run (all zero for FP64 couplings).  No counterpart

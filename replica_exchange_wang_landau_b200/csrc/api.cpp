@@ -343,7 +343,12 @@ wlg_status wlg_engine_set_staging_ring(wlg_engine* engine, int32_t entries) {
 
 wlg_status wlg_engine_inject_wait_timeout(wlg_engine* engine) {
     WLG_ENGINE_GUARD(engine)
-    return guarded([&] { engine->impl->inject_wait_timeout(); });
+    return guarded([&] { engine->impl->inject_wait_timeout(-1, 0); });
+}
+
+wlg_status wlg_engine_inject_wait_timeout_at(wlg_engine* engine, int64_t walker, uint32_t blocks) {
+    WLG_ENGINE_GUARD(engine)
+    return guarded([&] { engine->impl->inject_wait_timeout(walker, blocks); });
 }
 
 wlg_status wlg_engine_run(wlg_engine* engine, wlg_run_totals* totals) {

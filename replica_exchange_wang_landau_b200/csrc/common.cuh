@@ -346,11 +346,13 @@ struct DeviceParams {  // wl::WlParameters + the run_rewl intervals, on the devi
     int32_t inverse_time;
     int32_t nalivaiko;
     int32_t collect;
-    int32_t withhold_draws;  // failure injection: producers publish no draws (wlg_engine_inject_wait_timeout)
+    int32_t withhold_draws;  // failure injection, 0: none; n: a launch's draw warps publish n - 1 blocks of draws ...
     double round_trip_margin;
     uint64_t exchange_interval;
     uint64_t max_attempts;     // 0 = unlimited
     uint64_t seed;
+    int32_t withhold_walker;   // ... those of this walker, -1: of every walker
+    int32_t pad;
 };
 
 constexpr int kRepresentatives = 9;

@@ -499,8 +499,11 @@ void Engine::take_control(const Control& ctl) {
     if (ctl.error) throw WlgError(static_cast<wlg_status>(ctl.error), "device error");
 }
 
-void Engine::inject_wait_timeout() {
-    view_.p.withhold_draws = 1;
+void Engine::inject_wait_timeout(int64_t walker, uint32_t blocks) {
+    if (walker < -1 || walker >= static_cast<int64_t>(walkers_) || blocks > (1u << 30))
+        throw WlgError(WLG_ERR_INVALID_ARGUMENT, "invalid failure injection");
+    view_.p.withhold_draws = static_cast<int32_t>(blocks) + 1;
+    view_.p.withhold_walker = static_cast<int32_t>(walker);
     drop_graph();
 }
 
@@ -547,7 +550,7 @@ bool Engine::fused_epochs() {
                      : 0;
         if (fused_ && !d_fused_.ptr)
             d_fused_.allocate(sizeof(FusedSync) + 2 * walkers_ * sizeof(FusedMail) +
-                              2 * walkers_ * static_cast<uint64_t>(view_.max_window_bins) * sizeof(double));
+                              2 * walkers_ * static_cast<uint64_t>(view_.max_window_bins) * sizeof(FusedBin));
     }
     return fused_ != 0;
 }
@@ -577,7 +580,7 @@ void Engine::launch_epochs(uint64_t count) {
         fe.epochs = static_cast<uint32_t>(count);
         fe.sync = d_fused_.get<FusedSync>();
         fe.mail = reinterpret_cast<FusedMail*>(fe.sync + 1);
-        fe.mail_log_g = reinterpret_cast<double*>(fe.mail + 2 * walkers_);
+        fe.mail_bins = reinterpret_cast<FusedBin*>(fe.mail + 2 * walkers_);
         launch_ahead_epochs(view_, fe, stream_);
         return;
     }

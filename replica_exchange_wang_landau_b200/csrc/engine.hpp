@@ -198,11 +198,15 @@ struct alignas(16) FusedMail {  // a walker's configuration at an epoch's close
     double energy;
     int32_t bin, slot;
 };
+struct alignas(16) FusedBin {  // and its window's bins
+    double log_g;
+    uint32_t visits, active;
+};
 struct FusedEpochs {
     uint32_t epochs = 0;   // 0: one epoch without its exchange
     FusedSync* sync = nullptr;
     FusedMail* mail = nullptr;     // 2 x walkers
-    double* mail_log_g = nullptr;  // 2 x walkers x max_window_bins
+    FusedBin* mail_bins = nullptr; // 2 x walkers x max_window_bins
 };
 // Whether all of the engine's walkers can be resident at once (false too when the sweep does not serve it).
 bool ahead_epochs_fit(const EngineView& v);
@@ -301,9 +305,10 @@ class Engine {
     // the dense sweep's staging depth: 16 (four blocks of draws) or 32 (six), 0 = 16
     void set_staging_ring(int entries);
     int staging_ring() const;
-    // Failure injection for tests: from the next epoch on, the draw producers of the split and
-    // single-window sweeps publish nothing, so every walker's bounded wait runs out.
-    void inject_wait_timeout();
+    // Failure injection for tests: from the next epoch on, the draw warps of the look-ahead and
+    // single-window sweeps publish `blocks` blocks a launch (of one walker, -1: all) and no more, so
+    // that the walker's bounded wait runs out.
+    void inject_wait_timeout(int64_t walker, uint32_t blocks);
     uint64_t walkers() const { return walkers_; }
     uint64_t bins() const { return bins_; }
     uint64_t spins() const { return sys_.n; }

@@ -44,8 +44,11 @@
 // many epochs to a launch; 2458 sites, 32 x 8 walkers: 3.28 -> 0.97 ms per epoch of 2458 attempts.  The
 // rows an accepted flip reads, 224 MB an epoch at 8x8x8, come from L2 at 2.8 TB/s.
 //
-// All waits are bounded: on timeout the walker records WLG_ERR_TIMEOUT, every role leaves and no
-// state is written back.
+// All waits are bounded: on timeout the walker records WLG_ERR_TIMEOUT and every role leaves.  A launch of
+// one epoch then writes no state back.  In a launch of several, which has written fields and spins at each
+// epoch's end, the run ends with that epoch: every walker that made it writes the state it has, and one that
+// failed the state it had before the epoch (from what it left in its mailbox), so that a walker's
+// configuration, estimates and generator always belong together, as they do after epochs launched one by one.
 #include <type_traits>
 
 #include "engine.hpp"
@@ -86,11 +89,7 @@ constexpr uint32_t kEntUniform = 2u;  // the attempt consumed its acceptance uni
 constexpr uint32_t kEntStop = 4u;     // no attempt: the batch has ended (or failed)
 constexpr uint32_t kEntSkip = 8u;     // no attempt: the draw was rejected by bounded()
 
-struct alignas(16) BinRecord {  // one bin of the walker's window
-    double log_g;
-    uint32_t visits;  // of this batch
-    uint32_t active;
-};
+using BinRecord = FusedBin;  // one bin of the walker's window; visits: not in the histogram yet
 // A block's attempts: what the walker publishes of each, and (1/t stage) what each adds to log g;
 // both at eight bytes per attempt, so that one running address serves them.
 struct alignas(16) Attempts {
@@ -137,7 +136,8 @@ constexpr int kAheadIn = 2;   // block the look-ahead warp follows
 constexpr int kWalkerIn = 3;  // block the walker is in
 constexpr int kStop = 4;      // the walker has ended its last batch
 constexpr int kFail = 5;      // a bounded wait gave up
-constexpr int kFinal = 6;     // the flips handed to the field warps are the batch's last
+constexpr int kFinal = 6;     // the flips handed to the field warps are the batch's last (kFinalGood, kFinalFailed)
+constexpr uint32_t kFinalGood = 1u, kFinalFailed = 2u;
 constexpr int kGo = 1;        // epochs closed: (count << 2) | flags
 constexpr uint32_t kGoLeave = 1u, kGoReload = 2u, kGoGaveUp = 3u;  // (kGoGaveUp: leave, a role did not get the word)
 constexpr int kCount = 8;     // [8], [9]: flips of the two flip lists
@@ -333,8 +333,8 @@ struct EpochClose {
 
 // One walker's end of an epoch, by its warp: what the exchange kernel does for all pairs
 // (src/parallel.cpp:157-166, 410-421, src/wang_landau.cpp:483-508, and the termination test of
-// src/parallel.cpp:527-533).  Each walker leaves its energy, bin, slot and log g in a mailbox of the
-// epoch's parity and arrives at a grid-wide count; when all have arrived, the two walkers of a pair
+// src/parallel.cpp:527-533).  Each walker leaves its energy, bin, slot and bins in a mailbox of the
+// epoch's parity (the bins also for itself, should it fail in the next epoch) and arrives at a grid-wide count; when all have arrived, the two walkers of a pair
 // evaluate the same expression from the same numbers, so that no second barrier is needed.  A mailbox
 // is written again two epochs later, after every walker has arrived once more; the termination counts
 // rotate over three sets, the first walker clearing the set that is two epochs ahead.
@@ -346,9 +346,9 @@ __device__ __forceinline__ EpochClose close_epoch(const EngineView& v, const Fus
     const int walkers = v.walkers, wpw = v.walkers_per_window;
     FusedSync* sync = fe.sync;
     FusedMail* box = fe.mail + static_cast<size_t>(parity_box) * walkers;
-    double* box_g = fe.mail_log_g + static_cast<size_t>(parity_box) * walkers * v.max_window_bins;
-    if (v.windows > 1 && status == 0)
-        for (int i = lane; i < nbins; i += 32) box_g[static_cast<size_t>(w) * v.max_window_bins + i] = bins[i].log_g;
+    FusedBin* box_bins = fe.mail_bins + static_cast<size_t>(parity_box) * walkers * v.max_window_bins;
+    if (status == 0 && (v.windows > 1 || epochs < fe.epochs))
+        for (int i = lane; i < nbins; i += 32) box_bins[static_cast<size_t>(w) * v.max_window_bins + i] = bins[i];
     if (lane == 0) {
         if (status != 0 && atomicCAS(&v.ctl->error, 0, status) == 0) v.ctl->error_walker = w;
         box[w] = FusedMail{st.energy, st.cur_bin, st.slot};
@@ -415,9 +415,10 @@ __device__ __forceinline__ EpochClose close_epoch(const EngineView& v, const Fus
     const int mine = st.cur_bin, theirs = other.bin;
     if (mine < wb || mine >= we || theirs < wb || theirs >= we || mine < ob || mine >= oe || theirs < ob || theirs >= oe)
         return c;  // exchange_log_probability is -infinity
-    const double* other_g = box_g + static_cast<size_t>(partner) * v.max_window_bins;
+    const FusedBin* other_bins = box_bins + static_cast<size_t>(partner) * v.max_window_bins;
     const double own_mine = bins[mine - wb].log_g, own_theirs = bins[theirs - wb].log_g;
-    const double other_mine = __ldcg(other_g + (mine - ob)), other_theirs = __ldcg(other_g + (theirs - ob));
+    const double other_mine = __ldcg(&other_bins[mine - ob].log_g);
+    const double other_theirs = __ldcg(&other_bins[theirs - ob].log_g);
     // ga[x] - ga[y] + gb[y] - gb[x] with a the left walker, x its bin, y the right walker's
     const double logp = c.left ? own_mine - own_theirs + other_theirs - other_mine
                                : other_theirs - other_mine + own_mine - own_theirs;
@@ -448,6 +449,9 @@ struct EpochIo {
     int32_t rt_state;     // pilot statistics: of the books
     uint64_t trips;
     uint64_t epoch0, offered;
+    uint64_t rng[4];      // the generator at the last epoch's end, `draws` draws on
+    uint32_t draws;
+    int32_t good;         // the launch's last epoch was made: its state is to be written
 };
 
 // The end of an epoch, by the look-ahead warp: the walker's state, its check, the epoch's close with
@@ -455,8 +459,9 @@ struct EpochIo {
 // warp that does this, because a branch on the lane number (or a call) inside the loop that holds the
 // attempt loop costs every attempt: 85 -> 107 us per epoch of the 8x8x8 workload.
 __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& a, const FusedEpochs& fe, EpochIo* io,
-                                           WalkerState* st_s, BinRecord* bins, uint32_t* word, int w, int wb, int nbins,
-                                           uint32_t epochs, uint32_t settlers, int lane) {
+                                           WalkerState* st_s, BinRecord* bins, uint32_t* word, const uint64_t* generator,
+                                           uint32_t draws, int w, int wb, int nbins, uint32_t epochs, uint32_t settlers,
+                                           int lane) {
     const DeviceParams& P = v.p;
     const bool fused = fe.epochs != 0;
     // A look-ahead warp that has given up comes here ahead of the walker, whose own waits then run out, each
@@ -472,7 +477,8 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
     uint64_t offered = io->offered;
     const size_t boff = static_cast<size_t>(w) * static_cast<size_t>(v.grid.count) + static_cast<size_t>(wb);
     // the field warps have brought the fields up to date, in shared memory and in HBM
-    if (walker_ended != 0 || wait_at_least(word + kSettled, epochs * settlers, nullptr) != 0 || ld_relaxed(word + kFail) != 0) {
+    if (walker_ended != 0 || wait_at_least(word + kSettled, epochs * settlers, nullptr) != 0 ||
+        ld_relaxed(word + kFinal) != kFinalGood) {
         failed = true;
         if (status == 0) status = WLG_ERR_TIMEOUT;
     }
@@ -515,17 +521,26 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
             st.last_flatness = P.inverse_time ? hs.coverage : hs.min_over_mean;
             if (stats_ready(hs, st.stage, P)) warp_begin_next_iteration(st, v.hist + boff, nullptr, nbins, P, lane);
         }
+        if (lane < 4) io->rng[lane] = generator[lane];
+        io->draws = draws;
+    } else if (fused) {
+        // back to the epoch's start: the bins as this walker left them in its mailbox, or as the launch found
+        // them; the state, the generator and, in HBM, the fields and spins are those of that time still
+        const FusedBin* box = fe.mail_bins + (static_cast<size_t>((epochs - 1) & 1u) * v.walkers + w) * v.max_window_bins;
+        for (int i = lane; i < nbins; i += 32)
+            bins[i] = epochs > 1 ? box[i] : BinRecord{v.log_g[boff + i], 0u, v.active[boff + i] != 0 ? 1u : 0u};
     }
     bool leave = true, reload = false, done = false;
+    bool ended = failed;  // the run ends with a failure, this walker's or another's
     if (fused) {
         // every walker arrives with its configuration's energy and bin, and each pair's two walkers
         // then decide their exchange alike
         const EpochClose c = close_epoch(v, fe, epochs, w, wb, nbins, bins, st, epoch0 + epochs - 1,
                                          st.stage == kFrozen, at_limit, failed ? status : 0, lane);
-        failed = failed || c.status != 0;
+        ended = ended || c.status != 0;
         if (c.status > 1) status = c.status;
-        leave = failed || c.done || epochs == fe.epochs;
-        if (c.swapped && !failed) {
+        leave = ended || c.done || epochs == fe.epochs;
+        if (c.swapped) {
             st.energy = c.energy;
             st.cur_bin = c.bin;
             st.slot = c.slot;
@@ -543,12 +558,10 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
     __syncwarp();
     uint32_t flags = (leave ? kGoLeave : 0u) | (reload ? kGoReload : 0u);
     if (lane == 0) {
-        if (failed) {
-            st_relaxed(word + kFail, 1u);
-        } else {
-            *st_s = st;
-            word[kSlot] = static_cast<uint32_t>(st.slot);
-        }
+        if (ended) st_relaxed(word + kFail, 1u);
+        *st_s = st;  // (a failed epoch's is as it was)
+        word[kSlot] = static_cast<uint32_t>(st.slot);
+        io->good = failed ? 0 : 1;
         io->energy = st.energy;
         io->factor = st.factor;
         io->stage = st.stage;
@@ -565,8 +578,8 @@ __device__ __noinline__ uint32_t end_epoch(const EngineView& v, const WalkArgs& 
         if (flags & kGoLeave) st_release(word + kStop, 1u);
         if (fused && w == 0 && (flags & kGoLeave)) {
             v.ctl->exchange_attempted += offered;
-            v.ctl->epoch = epoch0 + epochs;
-            v.ctl->done = done || failed || flags == kGoGaveUp ? 1 : 0;
+            v.ctl->epoch = epoch0 + epochs - (ended ? 1u : 0u);  // (an epoch that failed somewhere is not counted)
+            v.ctl->done = done || ended || flags == kGoGaveUp ? 1 : 0;
         }
     }
     return __shfl_sync(kFull, flags, 0);
@@ -642,6 +655,7 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
         first.bin = escaped ? wb : ws->cur_bin;
         first.active = static_cast<uint32_t>(ws->active_count);
         first.epoch0 = ctl->epoch;
+        for (int k = 0; k < 4; ++k) first.rng[k] = ws->rng[k];
         *reinterpret_cast<EpochIo*>(smem + L.io) = first;
     }
     __syncthreads();
@@ -1031,15 +1045,14 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
         if (failed || ld_relaxed(word + kFail) != 0) {
             // (in a launch of several epochs the first error is there already, unless a role gave up since)
             if (lane == 0) record_error(ctl, io->status > 0 ? io->status : WLG_ERR_TIMEOUT, w);
-            return;
+            if (!fused && !io->good) return;
         }
         const uint32_t exchanged = io->exchanged;
         WalkerState st = *st_s;
-        // the generator after the draws consumed: the block's first state, k draws on
+        // the generator after the draws consumed: the block's first state, some draws on
         {
-            const uint64_t* m = reinterpret_cast<const uint64_t*>(slot_of(s) + SL.misc);
-            Rng rng{m[0], m[1], m[2], m[3]};
-            for (uint32_t d = 0; d < k; ++d) rng.next();
+            Rng rng{io->rng[0], io->rng[1], io->rng[2], io->rng[3]};
+            for (uint32_t d = 0; d < io->draws; ++d) rng.next();
             st.rng[0] = rng.s0;
             st.rng[1] = rng.s1;
             st.rng[2] = rng.s2;
@@ -1068,8 +1081,8 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
         const FastMod fm = v.site_mod;
         Rng first{ws->rng[0], ws->rng[1], ws->rng[2], ws->rng[3]};  // before the block's first draw
         int s = 0;
-        bool open = P.withhold_draws == 0;  // withheld (failure injection): the walker's wait runs out
-        for (uint32_t b = 0; open; ++b) {
+        const uint32_t most = blocks_published(P, w);  // failure injection: the walker's wait runs out
+        for (uint32_t b = 0; b < most; ++b) {
             if (b >= static_cast<uint32_t>(slots)) {  // the record's last readers: the walker and the look-ahead
                 const uint32_t need = b - static_cast<uint32_t>(slots) + 1;
                 int r = wait_at_least(word + kAheadIn, need, word + kStop);
@@ -1115,6 +1128,7 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
     } else if (role == 2) {
         // ---- look-ahead ----------------------------------------------------------------------
         const int barrier_threads = 32 + 32 * field_warps;
+        EpochIo* io = reinterpret_cast<EpochIo*>(smem + L.io);
         int s = 0, k = 0;
         uint32_t table = 0;
         uint32_t made = 0, n_acc = 0, last_acc = 0;  // attempts followed; accepted; attempts made at the last acceptance
@@ -1236,9 +1250,12 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
             fr.m = 0.0;
             fr.row = static_cast<uint64_t>(first_site) * static_cast<uint64_t>(ld) * sizeof(JT);
             if (pad) flips[32 * (lists & 1u) + lane] = fr;
+            // the epoch was made if the walker says so and its entries have been followed to the end; what this
+            // decides, the writes of fields, spins and state, all go by this one word
+            const bool good = last && !gave_up && *reinterpret_cast<volatile int32_t*>(&io->status) == 0;
             if (lane == 0) {
                 word[kCount + (lists & 1u)] = static_cast<uint32_t>(flips_made);
-                word[kFinal] = last ? 1u : 0u;
+                word[kFinal] = !last ? 0u : good ? kFinalGood : kFinalFailed;
                 if (gave_up) st_relaxed(word + kFail, 1u);
             }
             __syncwarp();
@@ -1259,7 +1276,7 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
             __syncwarp();
             if (last) {  // the epoch's end
                 ++epochs;
-                if (ld_relaxed(word + kFail) == 0) {
+                if (good) {
                     int4* to = reinterpret_cast<int4*>(v.spins + static_cast<size_t>(word[kSlot]) * ld);
                     for (int i = lane; i < (ld >> 4); i += 32) to[i] = reinterpret_cast<const int4*>(sp_s)[i];
                 }
@@ -1271,8 +1288,9 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
                 }
                 st_relaxed(word + kBoundary, 0u);
                 __syncwarp();
-                const uint32_t go = end_epoch(v, a, fe, reinterpret_cast<EpochIo*>(smem + L.io), st_s, bins, word, w, wb,
-                                              nbins, epochs, settlers, lane);
+                const uint32_t go = end_epoch(v, a, fe, io, st_s, bins, word,
+                                              reinterpret_cast<const uint64_t*>(rec + SL.misc), static_cast<uint32_t>(k), w,
+                                              wb, nbins, epochs, settlers, lane);
                 if (go & kGoLeave) break;
                 if (go & kGoReload) {
                     load_spins(static_cast<int>(word[kSlot]), lane, 32);
@@ -1370,9 +1388,10 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
             bar_sync(kBarList, barrier_threads);
             const FlipRecord* list = flips + 32 * (lists & 1u);
             const int n = static_cast<int>(word[kCount + (lists & 1u)]);
-            const bool last = word[kFinal] != 0;
+            const uint32_t final = word[kFinal];
+            const bool last = final != 0;
             // an epoch's end: the fields go to HBM as well
-            double2* out = last && ld_relaxed(word + kFail) == 0
+            double2* out = final == kFinalGood
                                ? reinterpret_cast<double2*>(v.fields + static_cast<size_t>(word[kSlot]) * ld)
                                : nullptr;
             // eight rows in flight, then the last flips by fours (the list is padded with m = 0); sixteen
@@ -1434,6 +1453,14 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
         }
         __syncwarp();
         if (st_s->rep_pending) represent();  // a replica exchange changed the configuration
+        bool complete = true;
+        auto save = [&]() {  // after an epoch that was made: should the next one fail, these are what it started from
+            if (!complete || !io->good) return;
+            for (int i = lane; i < nbins; i += 32) {
+                v.sqdisp[boff + i] = sq_s[i];
+                v.dsamples[boff + i] = ds_s[i];
+            }
+        };
         int s = 0, k = 0;
         uint32_t epochs = 0;
         for (uint32_t b = 0;;) {
@@ -1487,8 +1514,10 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
                 io->trips = trips;
             }
             settle(kSettled);
+            complete = complete && !gave_up;
             const uint32_t go = wait_go(++epochs);
             if (go & kGoLeave) break;
+            save();
             if (go & kGoReload) {
                 load_book_spins(static_cast<int>(word[kSlot]));
                 E = st_s->energy;
@@ -1498,11 +1527,9 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
             rt_state = st_s->rt_state;
             trips = st_s->round_trips;
         }
-        if (ld_relaxed(word + kFail) == 0)
-            for (int i = lane; i < nbins; i += 32) {
-                v.sqdisp[boff + i] = sq_s[i];
-                v.dsamples[boff + i] = ds_s[i];
-            }
+        bar_sync(0, static_cast<int>(blockDim.x));  // every role has left
+        save();
+        return;
     }
 
     bar_sync(0, static_cast<int>(blockDim.x));  // every role has left

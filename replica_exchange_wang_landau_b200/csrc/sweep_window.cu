@@ -142,8 +142,8 @@ __global__ void __launch_bounds__(64 * kWindowMaxWalkers, 1) sweep_window_kernel
         const FastMod fm = v.site_mod;
         Rng rng{st.rng[0], st.rng[1], st.rng[2], st.rng[3]};
         uint32_t produced = 0, timeout = 0;
-        // withhold_draws: publish nothing, so that the walkers' bounded waits run out
-        for (bool open = v.p.withhold_draws == 0; open;) {
+        // (under failure injection few or none, so that the walker's bounded wait runs out)
+        for (uint32_t left = blocks_published(v.p, w); left != 0; --left) {
             uint32_t go = 0;
             if (lane == 0) {
                 for (uint32_t polls = 0; polls < kWindowProducerPolls; ++polls) {

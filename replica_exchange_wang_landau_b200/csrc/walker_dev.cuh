@@ -264,6 +264,12 @@ __device__ __forceinline__ double window_lower(const EngineView& v, int wb) {
     return v.grid.minimum + static_cast<double>(wb) * v.grid.width;
 }
 
+// Blocks of draws that walker w's draw warp publishes in a launch: all but under failure injection.
+__device__ __forceinline__ uint32_t blocks_published(const DeviceParams& p, int w) {
+    const bool withheld = p.withhold_draws != 0 && (p.withhold_walker < 0 || p.withhold_walker == w);
+    return withheld ? static_cast<uint32_t>(p.withhold_draws) - 1u : ~0u;
+}
+
 __device__ __forceinline__ void record_error(Control* ctl, int status, int walker) {
     if (atomicCAS(&ctl->error, 0, status) == 0) ctl->error_walker = walker;
     ctl->done = 1;

@@ -642,11 +642,12 @@ class Engine:
         """The dense sweep's staging depth: 16 (four blocks of draws) or 32 (six); 0 = 16."""
         _check(self._lib.wlg_engine_set_staging_ring(self._h, int(entries)))
 
-    def inject_wait_timeout(self) -> None:
+    def inject_wait_timeout(self, walker: int = -1, blocks: int = 0) -> None:
         """Failure injection for tests: the draw warps of the look-ahead and single-window sweeps
         publish nothing from the next epoch on, so the walkers' bounded waits run out and the
-        next run call raises a DeviceError with status WLG_ERR_TIMEOUT."""
-        _check(self._lib.wlg_engine_inject_wait_timeout(self._h))
+        next run call raises a DeviceError with status WLG_ERR_TIMEOUT.  `walker`: that one's only;
+        `blocks`: after as many blocks of draws of a launch."""
+        _check(self._lib.wlg_engine_inject_wait_timeout_at(self._h, int(walker), int(blocks)))
 
     def set_launch(self, walkers_per_block: int = 0, epochs_per_graph: int = 0) -> None:
         _check(self._lib.wlg_engine_set_launch(self._h, int(walkers_per_block), int(epochs_per_graph)))
