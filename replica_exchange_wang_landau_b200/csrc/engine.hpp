@@ -12,6 +12,7 @@
 
 #include "../../include/wlg.h"
 #include "common.cuh"
+#include "shared_memory.hpp"
 
 namespace wlg {
 

@@ -445,13 +445,8 @@ using SweepFn = void (*)(EngineView, WalkArgs);
 
 template <int P>
 SweepFn sweep_fn() {
-    static bool configured = false;
-    if (!configured) {
-        check_cuda(cudaFuncSetAttribute(reinterpret_cast<const void*>(&sweep_dense_kernel<P>),
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
+    static SharedMemoryOptIn opt_in;
+    check_cuda(opt_in(reinterpret_cast<const void*>(&sweep_dense_kernel<P>)), "cudaFuncSetAttribute");
     return &sweep_dense_kernel<P>;
 }
 

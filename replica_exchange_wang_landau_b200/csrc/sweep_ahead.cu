@@ -1539,13 +1539,8 @@ using AheadFn = void (*)(EngineView, WalkArgs, int, int, FusedEpochs);
 
 template <int kPrec, bool kPow2, bool kAlone, bool kCollect>
 AheadFn ahead_fn() {
-    static bool configured = false;
-    if (!configured) {
-        check_cuda(cudaFuncSetAttribute(reinterpret_cast<const void*>(&sweep_ahead_kernel<kPrec, kPow2, kAlone, kCollect>),
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
+    static SharedMemoryOptIn opt_in;
+    check_cuda(opt_in(reinterpret_cast<const void*>(&sweep_ahead_kernel<kPrec, kPow2, kAlone, kCollect>)), "cudaFuncSetAttribute");
     return &sweep_ahead_kernel<kPrec, kPow2, kAlone, kCollect>;
 }
 

@@ -495,13 +495,8 @@ using SweepFn = void (*)(EngineView, WalkArgs);
 
 template <int kK, bool kPow2, int kPrec, bool kCollect>
 SweepFn csr_fn() {
-    static bool configured = false;
-    if (!configured) {
-        check_cuda(cudaFuncSetAttribute(reinterpret_cast<const void*>(&sweep_csr_kernel<kK, kPow2, kPrec, kCollect>),
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
+    static SharedMemoryOptIn opt_in;
+    check_cuda(opt_in(reinterpret_cast<const void*>(&sweep_csr_kernel<kK, kPow2, kPrec, kCollect>)), "cudaFuncSetAttribute");
     return &sweep_csr_kernel<kK, kPow2, kPrec, kCollect>;
 }
 

@@ -496,13 +496,8 @@ using WindowFn = void (*)(EngineView, uint32_t);
 
 template <bool kPow2>
 WindowFn window_fn() {
-    static bool configured = false;
-    if (!configured) {
-        check_cuda(cudaFuncSetAttribute(reinterpret_cast<const void*>(&sweep_window_kernel<kPow2>),
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
-                   "cudaFuncSetAttribute");
-        configured = true;
-    }
+    static SharedMemoryOptIn opt_in;
+    check_cuda(opt_in(reinterpret_cast<const void*>(&sweep_window_kernel<kPow2>)), "cudaFuncSetAttribute");
     return &sweep_window_kernel<kPow2>;
 }
 

@@ -536,12 +536,8 @@ using InitFn = void (*)(EngineView, InitArgs);
 
 template <int P, bool C, bool S, bool F>
 static void set_smem_attr(const void* fn) {
-    static bool done = false;
-    if (!done) {
-        check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024),
-                   "cudaFuncSetAttribute");
-        done = true;
-    }
+    static SharedMemoryOptIn opt_in;
+    check_cuda(opt_in(fn), "cudaFuncSetAttribute");
 }
 
 template <int P, bool C, bool S, bool F>
