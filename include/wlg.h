@@ -355,6 +355,9 @@ wlg_status wlg_engine_inject_wait_timeout(wlg_engine* engine);
  * middle of the launch.  Where epochs share a launch the run ends with the epoch in which that happens:
  * the other walkers have made it, the failed one has the state it had before it. */
 wlg_status wlg_engine_inject_wait_timeout_at(wlg_engine* engine, int64_t walker, uint32_t blocks);
+/* The sweep that runs the engine's epochs: "single-window", "look-ahead", "ring", "csr" or "generic"
+ * (NULL after an error).  Results do not depend on it.  No counterpart in the reference. */
+const char* wlg_engine_sweep(wlg_engine* engine);
 /* 1 when the engine runs its epochs with the single-window kernel, else 0. */
 int32_t wlg_engine_window_sweep(const wlg_engine* engine);
 /* The drift report of a mixed-precision run (all zero for FP64 couplings).  No counterpart

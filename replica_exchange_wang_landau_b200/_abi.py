@@ -318,6 +318,7 @@ SIGNATURES = {
     "wlg_engine_set_launch": (_i32, [_vp, _i32, _i32]),
     "wlg_engine_set_window_sweep": (_i32, [_vp, _i32]),
     "wlg_engine_window_sweep": (_i32, [_vp]),
+    "wlg_engine_sweep": (C.c_char_p, [_vp]),
     "wlg_engine_walkers": (_u64, [_vp]),
     "wlg_engine_bins": (_u64, [_vp]),
     "wlg_engine_spins": (_u64, [_vp]),

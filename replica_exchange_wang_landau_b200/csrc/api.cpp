@@ -431,6 +431,15 @@ wlg_status wlg_engine_set_window_sweep(wlg_engine* engine, int32_t enabled) {
     return guarded([&] { engine->impl->set_window_sweep(enabled != 0); });
 }
 
+const char* wlg_engine_sweep(wlg_engine* engine) {
+    const char* name = nullptr;
+    const auto ask = [&]() -> wlg_status {
+        WLG_ENGINE_GUARD(engine)
+        return guarded([&] { name = engine->impl->sweep(); });
+    };
+    return ask() == WLG_OK ? name : nullptr;
+}
+
 int32_t wlg_engine_window_sweep(const wlg_engine* engine) {
     return engine && engine->impl && engine->impl->window_sweep() ? 1 : 0;
 }

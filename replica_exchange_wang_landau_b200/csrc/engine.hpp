@@ -189,6 +189,7 @@ void launch_walk(const EngineView& v, const WalkArgs& a, int walkers_per_block, 
 // sweep_ahead.cu: the dense sweep; false when it does not serve the engine (the Nalivaiko mask, a
 // cutoff system without full rows, or a walker that does not fit in shared memory).
 bool launch_sweep_ahead(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
+bool sweep_ahead_serves(const EngineView& v);
 // Several epochs and their exchanges in one cooperative launch of that sweep.
 struct FusedSync {         // zeroed before each launch
     uint32_t arrived;      // walkers that have closed an epoch, counted on
@@ -212,12 +213,14 @@ struct FusedEpochs {
 // Whether all of the engine's walkers can be resident at once (false too when the sweep does not serve it).
 bool ahead_epochs_fit(const EngineView& v);
 void launch_ahead_epochs(const EngineView& v, const FusedEpochs& epochs, cudaStream_t stream);
-// sweep.cu: the dense sweep with the Nalivaiko mask or, where the look-ahead sweep does not fit, pilot
-// statistics; false when the walker does not fit the shared-memory ring, or has neither.
+// sweep.cu: the dense sweep with the Nalivaiko mask, and where the look-ahead sweep does not fit; false when
+// the walker does not fit the shared-memory ring either.
 bool launch_sweep_dense(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
+bool sweep_dense_serves(const EngineView& v);
 // The staging depths wlg_engine_set_staging_ring accepts for this engine (log2 of the staged draws).
 std::vector<int> split_ring_logs(const EngineView& v);
 bool launch_sweep_csr(const EngineView& v, const WalkArgs& a, int walkers_per_block, cudaStream_t stream);
+bool sweep_csr_serves(const EngineView& v);
 // sweep_window.cu: whole epochs of a single-window run of a dense FP64 system of at most 32
 // sites and 4 walkers, without pilot statistics or the Nalivaiko mask, in one launch
 bool window_sweep_fits(const EngineView& v);
@@ -310,6 +313,13 @@ class Engine {
     // single-window sweeps publish `blocks` blocks a launch (of one walker, -1: all) and no more, so
     // that the walker's bounded wait runs out.
     void inject_wait_timeout(int64_t walker, uint32_t blocks);
+    // the sweep that runs its epochs (wlg_engine_sweep)
+    const char* sweep() {
+        if (window_epochs()) return "single-window";
+        if (sweep_ahead_serves(view_)) return "look-ahead";
+        if (sweep_dense_serves(view_)) return "ring";
+        return sweep_csr_serves(view_) ? "csr" : "generic";
+    }
     uint64_t walkers() const { return walkers_; }
     uint64_t bins() const { return bins_; }
     uint64_t spins() const { return sys_.n; }

@@ -1,5 +1,5 @@
-// sweep.cu — the dense REWL sweep with the Nalivaiko mask, with or without pilot statistics (without
-// the mask: sweep_ahead.cu): WangLandauWalker::run_attempts / attempt_flip (src/wang_landau.cpp:244-315) for
+// sweep.cu — the dense REWL sweep with the Nalivaiko mask, and without it where a window is too wide for
+// sweep_ahead.cu: WangLandauWalker::run_attempts / attempt_flip (src/wang_landau.cpp:244-315) for
 // one batch of exchange_interval attempts, then the walker-local flatness / 1/t check of run_rewl
 // (src/parallel.cpp:395-407).
 //
@@ -76,7 +76,7 @@ __device__ __forceinline__ void issue_row(uint32_t dst, const void* src, uint32_
 struct RingLayout {
     size_t ring, bars, base, total;
 };
-__host__ __device__ inline RingLayout ring_layout(int ld, int mwb, size_t jbytes) {
+__host__ __device__ inline RingLayout ring_layout(int ld, int mwb, bool features, size_t jbytes) {
     RingLayout L;
     size_t at = 0;
     L.ring = at;
@@ -84,7 +84,7 @@ __host__ __device__ inline RingLayout ring_layout(int ld, int mwb, size_t jbytes
     L.bars = at;
     at += round16(kSlots * 8);
     L.base = at;
-    at += smem_layout(ld, mwb, true, true).total;
+    at += smem_layout(ld, mwb, true, features).total;
     L.total = at;
     return L;
 }
@@ -138,7 +138,7 @@ __device__ __forceinline__ void row_update(const void* row_smem, int ld, double 
     }
 }
 
-template <int kPrec>
+template <int kPrec, bool kFeat>
 __global__ void __launch_bounds__(32, 1) sweep_dense_kernel(EngineView v, WalkArgs a) {
     using JT = typename CouplingType<kPrec>::T;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -148,8 +148,8 @@ __global__ void __launch_bounds__(32, 1) sweep_dense_kernel(EngineView v, WalkAr
     Control* ctl = v.ctl;
     if (a.epoch_mode && *reinterpret_cast<volatile int32_t*>(&ctl->done)) return;
 
-    const RingLayout RL = ring_layout(v.ld, v.max_window_bins, sizeof(JT));
-    const SmemLayout L = smem_layout(v.ld, v.max_window_bins, true, true);
+    const RingLayout RL = ring_layout(v.ld, v.max_window_bins, kFeat, sizeof(JT));
+    const SmemLayout L = smem_layout(v.ld, v.max_window_bins, true, kFeat);
     unsigned char* base = smem + RL.base;
     const JT* ring_rows = reinterpret_cast<const JT*>(smem + RL.ring);
     double* f = reinterpret_cast<double*>(base + L.fields);
@@ -167,8 +167,8 @@ __global__ void __launch_bounds__(32, 1) sweep_dense_kernel(EngineView v, WalkAr
     double* fg = v.fields + static_cast<size_t>(st.slot) * v.ld;
     int8_t* sg = v.spins + static_cast<size_t>(st.slot) * v.ld;
     const DeviceParams& P = v.p;
-    const bool collect = P.collect;
-    const bool nalivaiko = P.nalivaiko;
+    const bool collect = kFeat && P.collect;
+    const bool nalivaiko = kFeat && P.nalivaiko;
 
     if (st.cur_bin < wb || st.cur_bin >= we) {  // "Walker escaped its energy window"
         if (lane == 0) record_error(ctl, WLG_ERR_ESCAPED, w);
@@ -244,7 +244,7 @@ __global__ void __launch_bounds__(32, 1) sweep_dense_kernel(EngineView v, WalkAr
         lg_s[b] = v.log_g[boff + b];
         h_s[b] = v.hist[boff + b];
         act_s[b] = v.active[boff + b];
-        ref_s[b] = v.refine[boff + b];
+        if constexpr (kFeat) ref_s[b] = v.refine[boff + b];
         if (collect) {
             sq_s[b] = v.sqdisp[boff + b];
             ds_s[b] = v.dsamples[boff + b];
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(32, 1) sweep_dense_kernel(EngineView v, WalkAr
         v.log_g[boff + b] = lg_s[b];
         v.hist[boff + b] = h_s[b];
         v.active[boff + b] = act_s[b];
-        v.refine[boff + b] = ref_s[b];
+        if constexpr (kFeat) v.refine[boff + b] = ref_s[b];
         if (collect) {
             v.sqdisp[boff + b] = sq_s[b];
             v.dsamples[boff + b] = ds_s[b];
@@ -443,11 +443,15 @@ __global__ void __launch_bounds__(32, 1) sweep_dense_kernel(EngineView v, WalkAr
 
 using SweepFn = void (*)(EngineView, WalkArgs);
 
-template <int P>
+template <int kPrec, bool kFeat>
 SweepFn sweep_fn() {
     static SharedMemoryOptIn opt_in;
-    check_cuda(opt_in(reinterpret_cast<const void*>(&sweep_dense_kernel<P>)), "cudaFuncSetAttribute");
-    return &sweep_dense_kernel<P>;
+    check_cuda(opt_in(reinterpret_cast<const void*>(&sweep_dense_kernel<kPrec, kFeat>)), "cudaFuncSetAttribute");
+    return &sweep_dense_kernel<kPrec, kFeat>;
+}
+size_t ring_bytes(const EngineView& v) {
+    const size_t jbytes = v.precision == WLG_PRECISION_FP64 ? 8 : v.precision == WLG_PRECISION_FP32 ? 4 : 2;
+    return ring_layout(v.ld, v.max_window_bins, v.p.collect || v.p.nalivaiko, jbytes).total;
 }
 
 }  // namespace
@@ -471,16 +475,22 @@ std::vector<int> split_ring_logs(const EngineView& v) {
     return out;
 }
 
+// Every dense engine that the look-ahead sweep does not take and that fits: the Nalivaiko mask, and windows of
+// more than about 10,000 bins, whose records of 16 bytes do not fit beside its 57 KB of tables (8x8x8 sites,
+// 11,500 bins, 8 walkers: 0.48 ms per epoch of 512 attempts, 0.61 in walk_kernel, which takes what is left).
+bool sweep_dense_serves(const EngineView& v) { return !v.csr && ring_bytes(v) <= 227 * 1024; }
+
 bool launch_sweep_dense(const EngineView& v, const WalkArgs& a, cudaStream_t stream) {
-    if (!v.p.collect && !v.p.nalivaiko) return false;
-    const size_t jbytes = v.precision == WLG_PRECISION_FP64 ? 8 : v.precision == WLG_PRECISION_FP32 ? 4 : 2;
-    const size_t bytes = ring_layout(v.ld, v.max_window_bins, jbytes).total;
-    if (bytes > 227 * 1024) return false;
+    if (!sweep_dense_serves(v)) return false;
+    const bool features = v.p.collect || v.p.nalivaiko;
     SweepFn fn;
-    if (v.precision == WLG_PRECISION_FP32) fn = sweep_fn<WLG_PRECISION_FP32>();
-    else if (v.precision == WLG_PRECISION_BF16) fn = sweep_fn<WLG_PRECISION_BF16>();
-    else fn = sweep_fn<WLG_PRECISION_FP64>();
-    fn<<<static_cast<unsigned>(a.count), 32, bytes, stream>>>(v, a);
+    if (v.precision == WLG_PRECISION_FP32)
+        fn = features ? sweep_fn<WLG_PRECISION_FP32, true>() : sweep_fn<WLG_PRECISION_FP32, false>();
+    else if (v.precision == WLG_PRECISION_BF16)
+        fn = features ? sweep_fn<WLG_PRECISION_BF16, true>() : sweep_fn<WLG_PRECISION_BF16, false>();
+    else
+        fn = features ? sweep_fn<WLG_PRECISION_FP64, true>() : sweep_fn<WLG_PRECISION_FP64, false>();
+    fn<<<static_cast<unsigned>(a.count), 32, ring_bytes(v), stream>>>(v, a);
     check_cuda(cudaGetLastError(), "sweep_dense_kernel");
     return true;
 }

@@ -1589,6 +1589,8 @@ AheadLaunch ahead_launch(const EngineView& v) {
 
 }  // namespace
 
+bool sweep_ahead_serves(const EngineView& v) { return ahead_launch(v).fn != nullptr; }
+
 bool launch_sweep_ahead(const EngineView& v, const WalkArgs& a, cudaStream_t stream) {
     const AheadLaunch l = ahead_launch(v);
     if (!l.fn) return false;

@@ -554,14 +554,19 @@ void launch_ell_fill(int n, int width, const int32_t* ptr, const int32_t* col, c
     check_cuda(cudaGetLastError(), "ell_fill_kernel");
 }
 
+static size_t csr_walker_bytes(const EngineView& v) {
+    return csr_sweep_layout(v.max_window_bins, v.ell_width, v.precision == WLG_PRECISION_FP32 ? 4 : 8, v.p.collect != 0).total;
+}
+
+bool sweep_csr_serves(const EngineView& v) {  // (the Nalivaiko mask: walk_kernel)
+    return v.csr && v.ell_width != 0 && !v.p.nalivaiko && csr_walker_bytes(v) <= 227 * 1024;
+}
+
 bool launch_sweep_csr(const EngineView& v, const WalkArgs& a, int walkers_per_block, cudaStream_t stream) {
-    if (!v.csr || v.ell_width == 0 || v.p.nalivaiko) return false;  // the Nalivaiko mask: walk_kernel
-    const bool collect = v.p.collect != 0;
-    SweepFn fn = collect ? pick_csr<true>(v) : pick_csr<false>(v);
+    if (!sweep_csr_serves(v)) return false;
+    SweepFn fn = v.p.collect ? pick_csr<true>(v) : pick_csr<false>(v);
     if (!fn) return false;
-    const int vbytes = v.precision == WLG_PRECISION_FP32 ? 4 : 8;
-    const size_t per_walker = csr_sweep_layout(v.max_window_bins, v.ell_width, vbytes, collect).total;
-    if (per_walker > 227 * 1024) return false;
+    const size_t per_walker = csr_walker_bytes(v);
     int wpb = walkers_per_block < 1 ? 1 : (walkers_per_block > 8 ? 8 : walkers_per_block);
     while (wpb > 1 && per_walker * static_cast<size_t>(wpb) > 227 * 1024) --wpb;
     const unsigned blocks = static_cast<unsigned>((a.count + wpb - 1) / wpb);

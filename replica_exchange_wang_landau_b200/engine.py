@@ -653,6 +653,15 @@ class Engine:
         _check(self._lib.wlg_engine_set_launch(self._h, int(walkers_per_block), int(epochs_per_graph)))
 
     @property
+    def sweep(self) -> str:
+        """The sweep that runs the engine's epochs: "single-window", "look-ahead", "ring", "csr" or "generic"
+        (results do not depend on it)."""
+        name = self._lib.wlg_engine_sweep(self._h)
+        if name is None:
+            raise DeviceError(1, self._lib.wlg_last_error().decode())
+        return name.decode()
+
+    @property
     def window_sweep(self) -> bool:
         """Whether the engine is run as a single-window one (one window, small dense FP64 system; many
         epochs per launch, those of at most 32 attempts in a kernel of their own).  Setting False selects the per-epoch kernels (same results)."""
