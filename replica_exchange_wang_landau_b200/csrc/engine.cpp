@@ -948,7 +948,7 @@ void Engine::autotune(uint64_t trial_epochs, wlg_autotune_report* out) {
     const int epgs[] = {4, 8, 16, 32, 64};
     // the dense sweep's staging depth where it serves the engine
     std::vector<int> rings;
-    for (int rl : split_ring_logs(view_)) rings.push_back(1 << rl);
+    for (int rl : staging_logs(view_)) rings.push_back(1 << rl);
     if (rings.empty()) rings.push_back(0);
     struct Candidate {
         int ring, wpb, epg;
@@ -1005,20 +1005,20 @@ void Engine::set_staging_ring(int entries) {
     else if (entries == 32) rl = 5;
     else if (entries != 0) throw WlgError(WLG_ERR_INVALID_ARGUMENT, "The staging ring holds 16 or 32 draws");
     if (rl != 0) {
-        const std::vector<int> ok = split_ring_logs(view_);
+        const std::vector<int> ok = staging_logs(view_);
         if (std::find(ok.begin(), ok.end(), rl) == ok.end())
             throw WlgError(WLG_ERR_INVALID_ARGUMENT,
                            "This engine's sweep has no staging ring of " + std::to_string(entries) + " draws");
     }
-    if (rl == view_.split_ring_log) return;
-    view_.split_ring_log = rl;
+    if (rl == view_.staging_log) return;
+    view_.staging_log = rl;
     fused_ = ahead_serves_ = -1;  // the walker's shared memory has changed
     drop_graph();
 }
 
 int Engine::staging_ring() const {
-    if (split_ring_logs(view_).empty()) return 0;
-    return 1 << (view_.split_ring_log == 5 ? 5 : 4);
+    if (staging_logs(view_).empty()) return 0;
+    return 1 << (view_.staging_log == 5 ? 5 : 4);
 }
 
 void Engine::totals(wlg_run_totals* out) {

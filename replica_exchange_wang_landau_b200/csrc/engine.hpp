@@ -218,7 +218,7 @@ void launch_ahead_epochs(const EngineView& v, const FusedEpochs& epochs, cudaStr
 bool launch_sweep_dense(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
 bool sweep_dense_serves(const EngineView& v);
 // The staging depths wlg_engine_set_staging_ring accepts for this engine (log2 of the staged draws).
-std::vector<int> split_ring_logs(const EngineView& v);
+std::vector<int> staging_logs(const EngineView& v);
 bool launch_sweep_csr(const EngineView& v, const WalkArgs& a, int walkers_per_block, cudaStream_t stream);
 bool sweep_csr_serves(const EngineView& v);
 // sweep_window.cu: whole epochs of a single-window run of a dense FP64 system of at most 32

@@ -456,25 +456,6 @@ size_t ring_bytes(const EngineView& v) {
 
 }  // namespace
 
-// The staging depths wlg_engine_set_staging_ring accepts (log2 of the draws staged ahead of the
-// walker): 16 or 32 draws for a dense system of at most 1024 sites without pilot statistics or the
-// Nalivaiko mask, when that many J rows and the walker's state would fit one CTA's shared memory;
-// empty otherwise.  The look-ahead sweep stages three or four block records accordingly.
-std::vector<int> split_ring_logs(const EngineView& v) {
-    std::vector<int> out;
-    const bool features = v.p.collect || v.p.nalivaiko;
-    if (v.csr || features || v.ld > 1024) return out;
-    const size_t jbytes = v.precision == WLG_PRECISION_FP64 ? 8 : v.precision == WLG_PRECISION_FP32 ? 4 : 2;
-    const size_t walker = smem_layout(v.ld, v.max_window_bins, true, false).total + 64 +
-                          round16(static_cast<size_t>(v.max_window_bins) * 4);
-    for (int rl = 4; rl <= 5; ++rl) {
-        const size_t q = size_t{1} << rl;
-        const size_t staged = q * round16(static_cast<size_t>(v.ld) * jbytes) + round16(q * 2) + q * 20;
-        if (staged + walker <= 227 * 1024) out.push_back(rl);
-    }
-    return out;
-}
-
 // Every dense engine that the look-ahead sweep does not take and that fits: the Nalivaiko mask, and windows of
 // more than about 10,000 bins, whose records of 16 bytes do not fit beside its 57 KB of tables (8x8x8 sites,
 // 11,500 bins, 8 walkers: 0.48 ms per epoch of 512 attempts, 0.61 in walk_kernel, which takes what is left).

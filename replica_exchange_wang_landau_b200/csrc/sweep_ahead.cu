@@ -1554,6 +1554,9 @@ AheadFn pick_ahead(bool pow2, bool alone, bool collect) {
     return collect ? pick_ahead<kPrec, true>(pow2, alone) : pick_ahead<kPrec, false>(pow2, alone);
 }
 
+// Block records made ahead of the walker for a staging depth of 2^log draws.
+int slots_of(int log) { return log == 5 ? kMaxSlots : kMinSlots; }
+
 // How the kernel is launched for an engine; fn is null when the sweep does not serve it.
 struct AheadLaunch {
     AheadFn fn = nullptr;
@@ -1567,8 +1570,7 @@ AheadLaunch ahead_launch(const EngineView& v) {
     const bool collect = v.p.collect != 0;
     if (v.csr && !v.rows64 && !v.rows32) return l;
     const bool scaled = v.precision == WLG_PRECISION_BF16;
-    l.slots = v.split_ring_log == 5 ? kMaxSlots : kMinSlots;
-    if (ahead_layout(v.ld, v.max_window_bins, scaled, l.slots, collect).total > 227 * 1024) l.slots = kMinSlots;
+    l.slots = slots_of(v.staging_log);
     l.bytes = ahead_layout(v.ld, v.max_window_bins, scaled, l.slots, collect).total;
     if (l.bytes > 227 * 1024) return l;
     int device = 0;
@@ -1588,6 +1590,17 @@ AheadLaunch ahead_launch(const EngineView& v) {
 }
 
 }  // namespace
+
+// The staging depths wlg_engine_set_staging_ring accepts (log2 of the draws): those whose block records fit
+// beside the walker, for dense systems of at most 1024 sites without pilot statistics or the Nalivaiko mask.
+std::vector<int> staging_logs(const EngineView& v) {
+    std::vector<int> out;
+    if (v.csr || v.p.collect || v.p.nalivaiko || v.ld > 1024) return out;
+    for (int log = 4; log <= 5; ++log)
+        if (ahead_layout(v.ld, v.max_window_bins, v.precision == WLG_PRECISION_BF16, slots_of(log), false).total <= 227 * 1024)
+            out.push_back(log);
+    return out;
+}
 
 bool sweep_ahead_serves(const EngineView& v) { return ahead_launch(v).fn != nullptr; }
 

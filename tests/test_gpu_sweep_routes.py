@@ -5,7 +5,7 @@ from __future__ import annotations
 import pytest
 
 from helpers import random_axes, results_equal
-from replica_exchange_wang_landau_b200.engine import Engine, Geometry, RunConfig, System, run_rewl
+from replica_exchange_wang_landau_b200.engine import Engine, Geometry, InvalidArgument, RunConfig, System, run_rewl
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +35,29 @@ def test_wide_windows(oracle, bins, sweep, precision):
                       seed=11, max_mcs=60, exchange_interval_mcs=2, check_interval_mcs=6)
         c.coupling_precision = precision
         _check(oracle, s, c, sweep)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "bf16"])
+def test_staging_depths_are_those_that_fit(oracle, precision):
+    """Six block records fit beside the walker wherever the look-ahead sweep has a staging depth; an engine whose
+    window is too wide for that sweep has none."""
+    s = _lattice((9, 10, 11), 4)
+    c = RunConfig(emin=-400, emax=400, bin_width=1.0, windows=2, walkers=2, seed=12, max_mcs=6,
+                  exchange_interval_mcs=1, check_interval_mcs=2)
+    c.coupling_precision = precision
+    c.resolve_mcs(s.size())
+    with Engine(s, c) as e:
+        assert e.sweep == "look-ahead"
+        e.set_staging_ring(32)
+        e.run()
+        got = e.result()
+    assert results_equal(got, oracle.run_rewl(s, c)) == []
+    s = _lattice((4, 4, 4), 3)
+    c = RunConfig(emin=-5750 * 2.0 ** -7, emax=5750 * 2.0 ** -7, bin_width=2.0 ** -7, windows=1, walkers=2, seed=11)
+    c.coupling_precision = precision
+    c.resolve_mcs(s.size())
+    with Engine(s, c) as e:
+        assert e.sweep == "ring"
+        for entries in (16, 32):
+            with pytest.raises(InvalidArgument):
+                e.set_staging_ring(entries)
