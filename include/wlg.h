@@ -320,8 +320,8 @@ typedef struct wlg_autotune_report {
     int32_t pad;
 } wlg_autotune_report;
 
-/* Launch-shape autotuner: times candidate shapes (walkers per CTA 1-8 for the generic sweep,
- * epochs per graph 4-64 (at least that many to a launch where epochs run many to a launch), the
+/* Launch-shape autotuner: times candidate shapes (walkers per CTA 1-8 for the CSR and generic sweeps,
+ * epochs per graph 4-64 unless the epochs share launches anyway, the
  * dense sweep's staging depth of 16 or 32 where it has one) on trial_epochs real epochs each through the product path
  * and keeps the fastest.  The shape never changes results, so the trial epochs count as epochs
  * of the run.  The exchange interval, which changes trajectories, is not tuned.  No

@@ -555,6 +555,12 @@ bool Engine::fused_epochs() {
     return fused_ != 0;
 }
 
+// Whether a launch takes as many epochs as make up some 2^18 attempts or more, whatever epochs_per_graph is.
+// (The host looks at checkpoints of all walkers and the progress line between launches, as often as asked.)
+bool Engine::epochs_share_launches() {
+    return window_sweep_ || (!checkpointing_all_ && cfg_.progress_interval_seconds <= 0.0 && fused_epochs());
+}
+
 // Whether the epochs of a single-window engine run in its own kernel.  That closes an epoch in about 1.3 us
 // within one CTA, and takes 0.23 to 0.32 us per attempt; the look-ahead sweep 4 to 5 us an epoch and 0.117
 // (bin widths that are no power of two: 0.29 and 0.14).  Measured, us per epoch, own kernel / look-ahead sweep:
@@ -675,8 +681,7 @@ void Engine::run_epochs(uint64_t max_epochs, uint64_t* epochs_run, int32_t* done
         uint64_t per_launch = static_cast<uint64_t>(epochs_per_graph);
         if (window_sweep_) per_launch = std::clamp<uint64_t>((uint64_t{1} << 20) / interval, 1, 4096);
         // a launch of several epochs: at least the configured number, about 2^18 attempts per walker
-        // (the host looks at checkpoints of all walkers and the progress line between launches, as often as asked)
-        else if (!checkpointing_all_ && cfg_.progress_interval_seconds <= 0.0 && fused_epochs())
+        else if (epochs_share_launches())
             per_launch = std::max(per_launch, std::min<uint64_t>((uint64_t{1} << 18) / interval, 4096));
         uint64_t chunk = std::min<uint64_t>(budget, per_launch);
         if (checkpointing_) {
@@ -929,24 +934,26 @@ void Engine::set_launch(int wpb, int epg) {
     if (wpb) drop_graph();
 }
 
-// Launch-shape autotuner: each candidate (staging depth of the dense sweep, walkers per CTA of
-// the generic sweep, epochs per graph replay) runs `trial_epochs` real epochs of this engine
-// through the product path after a warm-up replay that builds its graph, timed with device
-// events; the fastest per epoch is kept.  The candidates are timed twice, in order and then in
-// reverse order, and each one's two times are added: the cost of an epoch drifts as the run
+// Launch-shape autotuner: each candidate (staging depth of the look-ahead sweep, walkers per CTA of
+// the CSR and generic sweeps, epochs per graph replay) runs `trial_epochs` real epochs of this engine
+// through the product path after a warm-up run that builds its graph, timed with device
+// events; the fastest per epoch is kept.  Only what the engine's launches depend on is varied: where
+// epochs share launches of about 2^18 attempts there is no graph whose length matters, and a trial of a
+// graph's length would find the longest the quickest, because it has the fewest launches to its name.
+// The candidates are timed in order and in reverse order, equally often, and each one's
+// times are added: the cost of an epoch drifts as the run
 // moves on (acceptance, stage), and a drift that is linear over the trials adds the same to
 // every candidate's sum.  The launch shape never changes results, so the trial epochs are
 // ordinary epochs of the run.  (The exchange interval, which does change the sampled
 // trajectories, is left as configured.)
 void Engine::autotune(uint64_t trial_epochs, wlg_autotune_report* out) {
     if (trial_epochs == 0) throw WlgError(WLG_ERR_INVALID_ARGUMENT, "autotune needs at least one trial epoch");
-    const bool generic = sys_.csr || sys_.ld > 1024 || features_;
-    const int wpbs_generic[] = {1, 2, 4, 8};
-    const int wpbs_dense[] = {1};
-    const int* wpbs = generic ? wpbs_generic : wpbs_dense;
-    const int n_wpb = generic ? 4 : 1;
-    const int epgs[] = {4, 8, 16, 32, 64};
-    // the dense sweep's staging depth where it serves the engine
+    const bool shared = epochs_share_launches();
+    const bool per_cta = !window_epochs() && !sweep_ahead_serves(view_) && !sweep_dense_serves(view_);
+    const std::vector<int> wpbs = per_cta ? std::vector<int>{1, 2, 4, 8} : std::vector<int>{walkers_per_block};
+    const std::vector<int> epgs = shared ? std::vector<int>{epochs_per_graph} : std::vector<int>{4, 8, 16, 32, 64};
+    const int passes = shared ? 6 : 2;
+    // the look-ahead sweep's staging depth where it has one
     std::vector<int> rings;
     for (int rl : staging_logs(view_)) rings.push_back(1 << rl);
     if (rings.empty()) rings.push_back(0);
@@ -957,18 +964,18 @@ void Engine::autotune(uint64_t trial_epochs, wlg_autotune_report* out) {
     };
     std::vector<Candidate> cands;
     for (int ring : rings)
-        for (int a = 0; a < n_wpb; ++a)
-            for (int epg : epgs) cands.push_back({ring, wpbs[a], epg});
+        for (int wpb : wpbs)
+            for (int epg : epgs) cands.push_back({ring, wpb, epg});
     wlg_autotune_report r{};
-    for (int pass = 0; pass < 2; ++pass) {
+    for (int pass = 0; pass < passes; ++pass) {
         for (size_t k = 0; k < cands.size() && !done_; ++k) {
-            Candidate& c = cands[pass == 0 ? k : cands.size() - 1 - k];
+            Candidate& c = cands[pass % 2 == 0 ? k : cands.size() - 1 - k];
             if (c.ring) set_staging_ring(c.ring);
             set_launch(c.wpb, c.epg);
             wlg_epoch_timing t{};
-            time_run(static_cast<uint64_t>(c.epg), &t);  // builds and warms the graph
+            time_run(shared ? trial_epochs : static_cast<uint64_t>(c.epg), &t);  // builds and warms the graph
             const uint64_t rounds = std::max<uint64_t>(1, (trial_epochs + c.epg - 1) / c.epg);
-            time_run(rounds * c.epg, &t);
+            time_run(shared ? trial_epochs : rounds * c.epg, &t);
             ++r.trials;
             if (t.epochs == 0) continue;
             c.ms += t.total_ms / static_cast<double>(t.epochs);

@@ -397,6 +397,7 @@ class Engine {
     static constexpr uint64_t kFusedEpochAttempts = 1u << 17;
     bool fused_epochs();
     bool window_epochs();
+    bool epochs_share_launches();
     // Cutoff systems of at most this many sites and at most four walkers per SM run in the look-ahead
     // sweep on a copy of their couplings as full rows; a row's zeros change no field (a field is
     // never -0.0).  The CSR sweep is bound by each walker's memory latency and needs about a

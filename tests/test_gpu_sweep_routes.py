@@ -61,3 +61,29 @@ def test_staging_depths_are_those_that_fit(oracle, precision):
         for entries in (16, 32):
             with pytest.raises(InvalidArgument):
                 e.set_staging_ring(entries)
+
+
+AUTOTUNE = {  # (cutoff, pilot statistics, Nalivaiko mask, sweep, candidates, passes)
+    "dense": (0.0, False, False, "look-ahead", 2, 6),  # the two staging depths
+    "pilot": (0.0, True, False, "look-ahead", 1, 6),
+    "cutoff": (1.8, False, False, "look-ahead", 1, 6),
+    "mask": (0.0, False, True, "ring", 5, 2),  # epochs per graph replay
+    "cutoff_mask": (1.8, False, True, "generic", 20, 2),  # ... and walkers per CTA
+}
+
+
+@pytest.mark.parametrize("name", list(AUTOTUNE))
+def test_autotune_varies_what_the_launches_depend_on(name):
+    cutoff, pilot, mask, sweep, candidates, passes = AUTOTUNE[name]
+    s = _lattice((4, 4, 4), 3, cutoff)
+    c = RunConfig(emin=-60, emax=60, bin_width=0.5, windows=2, walkers=2, overlap=0.5, seed=9)
+    c.wl.collect_window_statistics, c.wl.nalivaiko_mod = pilot, mask
+    c.wl.inverse_time_enabled = not mask
+    c.exchange_interval_mcs, c.max_mcs = 2.0, 1e6
+    c.resolve_mcs(s.size())
+    with Engine(s, c) as e:
+        assert e.sweep == sweep
+        e.set_launch(0, 10)
+        r = e.autotune(4)
+        assert r["trials"] == candidates * passes and r["ms_per_epoch"] > 0
+        assert (r["epochs_per_graph"] == 10) == (passes == 6)
