@@ -583,11 +583,13 @@ void Engine::launch_epochs(uint64_t count) {
     }
     if (fused_epochs()) {
         FusedEpochs fe;
-        fe.epochs = static_cast<uint32_t>(count);
         fe.sync = d_fused_.get<FusedSync>();
         fe.mail = reinterpret_cast<FusedMail*>(fe.sync + 1);
         fe.mail_bins = reinterpret_cast<FusedBin*>(fe.mail + 2 * walkers_);
-        launch_ahead_epochs(view_, fe, stream_);
+        for (; count > 0; count -= fe.epochs) {  // (launches after the run's end do nothing)
+            fe.epochs = static_cast<uint32_t>(std::min(count, most_shared_epochs(p_.exchange_interval)));
+            launch_ahead_epochs(view_, fe, stream_);
+        }
         return;
     }
     WalkArgs a{};

@@ -210,6 +210,11 @@ struct FusedEpochs {
     FusedMail* mail = nullptr;     // 2 x walkers
     FusedBin* mail_bins = nullptr; // 2 x walkers x max_window_bins
 };
+// The most epochs of so many attempts in one launch: a bin's visits are counted in 32 bits until a check or the
+// launch's end adds them to the histogram.
+constexpr uint64_t most_shared_epochs(uint64_t interval) {
+    return interval < 0xffffffffULL ? 0xffffffffULL / (interval == 0 ? 1 : interval) : 1;
+}
 // Whether all of the engine's walkers can be resident at once (false too when the sweep does not serve it).
 bool ahead_epochs_fit(const EngineView& v);
 void launch_ahead_epochs(const EngineView& v, const FusedEpochs& epochs, cudaStream_t stream);

@@ -72,6 +72,18 @@ def test_opened_by_staying(tmp_path):
     assert res.returncode == 0 and res.stdout.startswith("ok"), res.stdout
 
 
+def test_visits_of_a_launch_fit_their_counter(tmp_path):
+    exe = tmp_path / "shared_epochs_check"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I/usr/local/cuda/include",
+                    str(ROOT / "tests" / "native" / "shared_epochs_check.cpp"), "-o", str(exe), "-L/usr/local/cuda/lib64",
+                    "-lcudart"], check=True)
+    res = subprocess.run([str(exe)], capture_output=True, text=True, env={"LD_LIBRARY_PATH": "/usr/local/cuda/lib64"})
+    assert res.returncode == 0 and res.stdout == "ok\n", res.stdout
+    engine = (ROOT / "replica_exchange_wang_landau_b200" / "csrc" / "engine.cpp").read_text()
+    launch = engine[engine.index("void Engine::launch_epochs("):engine.index("void Engine::maybe_checkpoint(")]
+    assert "std::min(count, most_shared_epochs(p_.exchange_interval))" in launch
+
+
 def _epoch_end(replaces: bool, waiting: int = 2):
     """All outcomes of an epoch's end: `waiting` roles that look at the word at any time and give up at any
     later one, against the look-ahead warp that publishes "go on" at any time.  The word is 0 until then;
