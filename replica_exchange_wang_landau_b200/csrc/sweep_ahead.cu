@@ -1467,8 +1467,11 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
             const int32_t* sites = reinterpret_cast<const int32_t*>(slot_of(s) + SL.site);
             const Attempts* block = attempts + (b & 1u);
             int e = 0;
-            bool stop = false, gave_up = false;
-            while (k < kStep) {
+            // The look-ahead warp clears this buffer of the entries of two blocks before when it is through with
+            // the last block, which is later than here where its fields come late (two walkers to an SM,
+            // or thousands of sites).
+            bool stop = wait_at_least(word + kAheadIn, b, word + kStop) == 2, gave_up = stop;
+            while (!stop && k < kStep) {
                 uint32_t x = ld_relaxed(&block->entry[e].x);
                 for (uint32_t polls = 0; x == 0 && polls < kPolls; ++polls) {
                     x = ld_relaxed(&block->entry[e].x);

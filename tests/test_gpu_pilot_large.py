@@ -1,0 +1,43 @@
+"""Pilot statistics in the look-ahead sweep (csrc/sweep_ahead.cu) where the fields of a block come later than its
+entries: two walkers to an SM, and thousands of sites.  Runs with squared displacements, samples, round trips and
+representatives, bit for bit against the CPU oracle."""
+from __future__ import annotations
+
+import pytest
+
+from helpers import random_axes, results_equal
+from replica_exchange_wang_landau_b200.engine import Engine, Geometry, RunConfig, System, run_rewl
+
+pytestmark = pytest.mark.gpu
+
+CASES = {  # dimensions, cutoff, windows, walkers, reach, width, couplings, attempts per epoch, epochs
+    "two_to_an_sm": ((8, 8, 8), 0.0, 32, 8, 190.0, 0.5, "fp64", 512, 12),
+    "two_to_an_sm_width": ((8, 8, 8), 0.0, 32, 8, 190.0, 0.4, "fp64", 301, 12),
+    "two_to_an_sm_fp32": ((8, 8, 8), 0.0, 32, 8, 190.0, 0.5, "fp32", 512, 8),
+    "two_to_an_sm_bf16": ((8, 8, 8), 0.0, 32, 8, 190.0, 0.5, "bf16", 512, 8),
+    "more_than_two": ((8, 8, 8), 0.0, 32, 12, 190.0, 0.5, "fp64", 512, 8),
+    "cutoff": ((10, 10, 10), 2.2, 32, 16, 200.0, 0.5, "fp64", 500, 6),
+    "sites_4096": ((16, 16, 16), 0.0, 2, 2, 300.0, 1.0, "fp64", 2000, 6),
+    "sites_4913": ((17, 17, 17), 0.0, 1, 2, 300.0, 0.75, "fp64", 2000, 6),
+}
+
+
+@pytest.mark.parametrize("name", list(CASES))
+def test_pilot_runs(oracle, name):
+    dims, cutoff, windows, walkers, reach, width, precision, interval, epochs = CASES[name]
+    g = Geometry.simple_cubic(*dims, periodic=True)
+    g.axes = random_axes(g.size(), 19)
+    s = System(g, 1.0, cutoff)
+    half = round(reach / width)
+    c = RunConfig(emin=-half * width, emax=half * width, bin_width=width, windows=windows, walkers=walkers, seed=20,
+                  overlap=0.75)
+    c.exchange_interval_uses_mcs = c.check_interval_uses_mcs = c.max_limit_uses_mcs = False
+    c.exchange_interval_attempts, c.wl.check_interval_attempts, c.max_attempts = interval, 4 * interval, epochs * interval
+    c.wl.collect_window_statistics = True
+    c.coupling_precision, c.recompute_interval_mcs = precision, 0.0
+    c.resolve_mcs(s.size())
+    with Engine(s, c) as e:
+        assert e.sweep == "look-ahead"
+    got = run_rewl(s, c)
+    assert results_equal(got, oracle.run_rewl(s, c)) == []
+    assert len(got.representatives) >= windows * walkers

@@ -137,3 +137,54 @@ def test_the_epochs_end_waits_for_the_walker():
     walker = SOURCE[SOURCE.index("// ---- the walker ---"):SOURCE.index("// ---- draws ---")]
     end = walker[walker.index("io->energy = E;"):]
     assert end.index("io->batch = batch;") < end.index("st_release(word + kEnded, epochs)") < end.index("kEntStop")
+
+
+def _books_read(waits: bool, ahead_delay: int, blocks: int = 12, per_block: int = 3) -> list:
+    """Walker, look-ahead warp and books over `blocks` blocks of `per_block` entries in two buffers, the
+    look-ahead warp `ahead_delay` steps behind in every block (its fields come late): the blocks whose entries
+    the books have read for each block.  `waits`: the books enter a block after the look-ahead warp has."""
+    entry = [[None] * per_block, [None] * per_block]
+    walker = {"b": 0, "e": 0}
+    ahead = {"b": 0, "late": ahead_delay}
+    books = {"b": 0, "e": 0}
+    handed, booked, read = 0, 0, []
+    for _ in range(10000):
+        if walker["b"] < blocks:
+            if walker["e"] < per_block:
+                entry[walker["b"] & 1][walker["e"]] = walker["b"]
+                walker["e"] += 1
+            elif handed > walker["b"]:
+                walker = {"b": walker["b"] + 1, "e": 0}
+        if books["b"] < blocks and (not waits or ahead["b"] >= books["b"]):
+            x = entry[books["b"] & 1][books["e"]]
+            if x is not None:
+                read.append((books["b"], x))
+                books["e"] += 1
+                if books["e"] == per_block:
+                    books = {"b": books["b"] + 1, "e": 0}
+                    booked = books["b"]
+        if ahead["b"] < blocks and entry[ahead["b"] & 1][-1] == ahead["b"]:
+            if ahead["late"]:
+                ahead["late"] -= 1
+            elif ahead["b"] == 0 or booked >= ahead["b"]:
+                if ahead["b"]:
+                    entry[(ahead["b"] + 1) & 1] = [None] * per_block
+                handed = ahead["b"] + 1
+                ahead = {"b": ahead["b"] + 1, "late": ahead_delay}
+        if books["b"] == blocks:
+            break
+    return read
+
+
+def test_the_books_read_the_entries_of_their_own_block():
+    for delay in range(12):
+        read = _books_read(True, delay)
+        assert len(read) == 36 and all(b == x for b, x in read), delay
+    # the model is not vacuous: books that do not wait read the entries of two blocks before
+    assert any(b != x for b, x in _books_read(False, 8))
+
+
+def test_the_books_wait_for_the_look_ahead_warp():
+    books = SOURCE[SOURCE.index("// ---- the books: pilot statistics"):]
+    loop = books[books.index("for (uint32_t b = 0;;) {"):]
+    assert loop.index("wait_at_least(word + kAheadIn, b, word + kStop)") < loop.index("block->entry[e].x")
