@@ -379,6 +379,7 @@ struct EngineView {
     int32_t spins_global;          // the generic sweep and the initialisation read spins from HBM
     const double* rows64;          // couplings as full rows for the look-ahead sweep (n x ld): J64 / J32, or
     const float* rows32;           // a copy of a small cutoff system's, zeros included; null: not served
+    int32_t split_sweep;           // the split sweep runs the engine (split_sweep_better, decided once)
     int32_t staging_log;        // staging depth of the dense sweep as log2 of 16 or 32 draws (4 or 5; 0 = 4)
     Grid grid;
     int32_t walkers;

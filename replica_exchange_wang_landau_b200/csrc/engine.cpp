@@ -335,6 +335,7 @@ void Engine::initialise_walkers(const wlg_run_config& c) {
     if (sys_.csr && !smem_fields_ && walker_smem_bytes(v, false, features_) > 200 * 1024) v.spins_global = 1;
     if (!sys_.csr && !fields_fit_in_smem(v, features_))
         throw WlgError(WLG_ERR_INVALID_ARGUMENT, "Dense system too large for the shared-memory walker (use a cutoff)");
+    v.split_sweep = split_sweep_better(v, sms, recompute_epochs_ == 1) ? 1 : 0;
     window_sweep_eligible_ = window_sweep_fits(v);
     window_sweep_ = window_sweep_eligible_;
 

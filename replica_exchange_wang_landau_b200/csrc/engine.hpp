@@ -186,10 +186,15 @@ size_t walker_smem_bytes(const EngineView& v, bool smem_fields, bool features);
 bool fields_fit_in_smem(const EngineView& v, bool features);
 void launch_init(const EngineView& v, const InitArgs& a, int walkers_per_block, cudaStream_t stream);
 void launch_walk(const EngineView& v, const WalkArgs& a, int walkers_per_block, cudaStream_t stream);
+// sweep_split.cu: the dense sweep of many walkers of a small system; false for other engines.
+bool launch_sweep_split(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
+// Whether that sweep is to run an engine; epochs_alone: its epochs are launched one by one.
+bool split_sweep_better(const EngineView& v, int sms, bool epochs_alone);
 // sweep_ahead.cu: the dense sweep; false when it does not serve the engine (the Nalivaiko mask, a
 // cutoff system without full rows, or a walker that does not fit in shared memory).
 bool launch_sweep_ahead(const EngineView& v, const WalkArgs& a, cudaStream_t stream);
 bool sweep_ahead_serves(const EngineView& v);
+int ahead_resident(const EngineView& v);  // walkers that fit on the GPU at once, 0: not served
 // Several epochs and their exchanges in one cooperative launch of that sweep.
 struct FusedSync {         // zeroed before each launch
     uint32_t arrived;      // walkers that have closed an epoch, counted on
@@ -321,6 +326,7 @@ class Engine {
     // the sweep that runs its epochs (wlg_engine_sweep)
     const char* sweep() {
         if (window_epochs()) return "single-window";
+        if (view_.split_sweep) return "split";
         if (sweep_ahead_serves(view_)) return "look-ahead";
         if (sweep_dense_serves(view_)) return "ring";
         return sweep_csr_serves(view_) ? "csr" : "generic";

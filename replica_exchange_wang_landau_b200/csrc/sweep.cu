@@ -24,6 +24,7 @@
 // The arithmetic is the reference's, operation for operation (see walker.cu for the shared
 // argument about fma(m, J, h) with m = +-2 and the power-of-two bin width).
 #include "engine.hpp"
+#include "row_copies.cuh"
 #include "walker_dev.cuh"
 
 namespace wlg {
@@ -33,18 +34,6 @@ namespace {
 constexpr int kSlots = 4;
 constexpr uint32_t kWaitPolls = 1u << 18;
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) {
-    return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-    uint32_t ok;
-    asm volatile(
-        "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n selp.u32 %0, 1, 0, p;\n}"
-        : "=r"(ok)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return ok != 0;
-}
 // Warp-uniform bounded wait for the completion of phase `parity` of one barrier.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     if (__all_sync(kFull, mbar_try(bar, parity))) return true;
@@ -88,11 +77,6 @@ __host__ __device__ inline RingLayout ring_layout(int ld, int mwb, bool features
     L.total = at;
     return L;
 }
-
-template <int kPrec> struct CouplingType;
-template <> struct CouplingType<WLG_PRECISION_FP64> { using T = double; };
-template <> struct CouplingType<WLG_PRECISION_FP32> { using T = float; };
-template <> struct CouplingType<WLG_PRECISION_BF16> { using T = __nv_bfloat16; };
 
 // fields[j] += m * row[j] (add_flip_delta, src/physics.cpp:190-195) from a row in shared
 // memory; m * row[j] is exact (m = +-2, times the BF16 row scale), so fma rounds once as

@@ -1569,7 +1569,7 @@ struct AheadLaunch {
 };
 AheadLaunch ahead_launch(const EngineView& v) {
     AheadLaunch l;
-    if (v.p.nalivaiko) return l;
+    if (v.p.nalivaiko || v.split_sweep) return l;
     const bool collect = v.p.collect != 0;
     if (v.csr && !v.rows64 && !v.rows32) return l;
     const bool scaled = v.precision == WLG_PRECISION_BF16;
@@ -1599,6 +1599,7 @@ AheadLaunch ahead_launch(const EngineView& v) {
 std::vector<int> staging_logs(const EngineView& v) {
     std::vector<int> out;
     if (v.csr || v.p.collect || v.p.nalivaiko || v.ld > 1024) return out;
+    if (v.split_sweep) return {4, 5};
     for (int log = 4; log <= 5; ++log)
         if (ahead_layout(v.ld, v.max_window_bins, v.precision == WLG_PRECISION_BF16, slots_of(log), false).total <= 227 * 1024)
             out.push_back(log);
@@ -1615,14 +1616,16 @@ bool launch_sweep_ahead(const EngineView& v, const WalkArgs& a, cudaStream_t str
     return true;
 }
 
-bool ahead_epochs_fit(const EngineView& v) {
+bool ahead_epochs_fit(const EngineView& v) { return v.walkers <= ahead_resident(v); }
+
+int ahead_resident(const EngineView& v) {
     const AheadLaunch l = ahead_launch(v);
-    if (!l.fn) return false;
+    if (!l.fn) return 0;
     int per_sm = 0;
     check_cuda(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, reinterpret_cast<const void*>(l.fn),
                                                              static_cast<int>(l.threads), l.bytes),
                "cudaOccupancyMaxActiveBlocksPerMultiprocessor");
-    return v.walkers <= per_sm * l.sms;
+    return per_sm * l.sms;
 }
 
 void launch_ahead_epochs(const EngineView& v, const FusedEpochs& epochs, cudaStream_t stream) {

@@ -586,6 +586,7 @@ static bool features_of(const EngineView& v) { return v.p.collect || v.p.nalivai
 
 void launch_walk(const EngineView& v, const WalkArgs& a, int wpb, cudaStream_t stream) {
     const bool features = features_of(v);
+    if (launch_sweep_split(v, a, stream)) return;  // sweep_split.cu: many walkers of a small system
     if (launch_sweep_ahead(v, a, stream)) return;  // sweep_ahead.cu: look-ahead blocks of draws
     if (!v.csr && launch_sweep_dense(v, a, stream)) return;  // sweep.cu: the TMA row ring
     if (v.csr && launch_sweep_csr(v, a, wpb, stream)) return;  // sweep_csr.cu: ELLPACK rows, fields in HBM
