@@ -1469,8 +1469,9 @@ __global__ void __launch_bounds__(32 * warps_for((kAlone ? kMaxRoles : kMaxRoles
             int e = 0;
             // The look-ahead warp clears this buffer of the entries of two blocks before when it is through with
             // the last block, which is later than here where its fields come late (two walkers to an SM,
-            // or thousands of sites).
-            bool stop = wait_at_least(word + kAheadIn, b, word + kStop) == 2, gave_up = stop;
+            // or thousands of sites).  It enters every block that the walker has ended, also after the walker
+            // has stopped.
+            bool stop = wait_at_least(word + kAheadIn, b, nullptr) != 0, gave_up = stop;
             while (!stop && k < kStep) {
                 uint32_t x = ld_relaxed(&block->entry[e].x);
                 for (uint32_t polls = 0; x == 0 && polls < kPolls; ++polls) {

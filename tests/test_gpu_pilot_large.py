@@ -41,3 +41,22 @@ def test_pilot_runs(oracle, name):
     got = run_rewl(s, c)
     assert results_equal(got, oracle.run_rewl(s, c)) == []
     assert len(got.representatives) >= windows * walkers
+
+
+@pytest.mark.parametrize("windows, walkers, interval", [(32, 16, 64), (32, 16, 512), (32, 8, 64), (32, 4, 64)])
+def test_every_attempt_is_a_sample(windows, walkers, interval):
+    """Long runs, epochs launched one by one (more walkers than fit on the GPU at once) and many to a launch: each
+    attempt adds one displacement sample, whatever the epochs' ends and the blocks' ends fall on."""
+    g = Geometry.simple_cubic(8, 8, 8, periodic=True)
+    g.axes = random_axes(512, 19)
+    s = System(g)
+    c = RunConfig(emin=-190.0, emax=190.0, bin_width=0.5, windows=windows, walkers=walkers, seed=21, overlap=0.75)
+    c.exchange_interval_uses_mcs, c.exchange_interval_attempts, c.max_mcs = False, interval, 0.0
+    c.wl.collect_window_statistics = True
+    c.resolve_mcs(512)
+    epochs = 1600 if interval == 64 else 400
+    with Engine(s, c) as e:
+        for _ in range(4):
+            e.run_epochs(epochs // 4)
+        samples = sum(int(e.sampling_statistics(w).displacement_samples.sum()) for w in range(windows))
+        assert samples == e.totals()["attempted"] == epochs * interval * windows * walkers

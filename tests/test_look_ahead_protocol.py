@@ -139,23 +139,26 @@ def test_the_epochs_end_waits_for_the_walker():
     assert end.index("io->batch = batch;") < end.index("st_release(word + kEnded, epochs)") < end.index("kEntStop")
 
 
-def _books_read(waits: bool, ahead_delay: int, blocks: int = 12, per_block: int = 3) -> list:
+def _books_read(waits: str, ahead_delay: int, blocks: int = 12, per_block: int = 3) -> list:
     """Walker, look-ahead warp and books over `blocks` blocks of `per_block` entries in two buffers, the
     look-ahead warp `ahead_delay` steps behind in every block (its fields come late): the blocks whose entries
-    the books have read for each block.  `waits`: the books enter a block after the look-ahead warp has."""
+    the books have read for each block.  The walker ends its batch with the last block's last draw and then
+    says that it has stopped.  `waits`: the books enter a block after the look-ahead warp has ("always"), or
+    so unless the walker has stopped ("until stop"), or at once ("")."""
     entry = [[None] * per_block, [None] * per_block]
     walker = {"b": 0, "e": 0}
     ahead = {"b": 0, "late": ahead_delay}
     books = {"b": 0, "e": 0}
-    handed, booked, read = 0, 0, []
+    handed, booked, read, stopped = 0, 0, [], False
     for _ in range(10000):
         if walker["b"] < blocks:
             if walker["e"] < per_block:
                 entry[walker["b"] & 1][walker["e"]] = walker["b"]
                 walker["e"] += 1
+                stopped = walker == {"b": blocks - 1, "e": per_block}
             elif handed > walker["b"]:
                 walker = {"b": walker["b"] + 1, "e": 0}
-        if books["b"] < blocks and (not waits or ahead["b"] >= books["b"]):
+        if not waits or ahead["b"] >= books["b"] or (waits == "until stop" and stopped):
             x = entry[books["b"] & 1][books["e"]]
             if x is not None:
                 read.append((books["b"], x))
@@ -163,6 +166,8 @@ def _books_read(waits: bool, ahead_delay: int, blocks: int = 12, per_block: int 
                 if books["e"] == per_block:
                     books = {"b": books["b"] + 1, "e": 0}
                     booked = books["b"]
+            elif books["b"] == blocks and stopped:
+                break  # the batch ended with the last block
         if ahead["b"] < blocks and entry[ahead["b"] & 1][-1] == ahead["b"]:
             if ahead["late"]:
                 ahead["late"] -= 1
@@ -171,20 +176,20 @@ def _books_read(waits: bool, ahead_delay: int, blocks: int = 12, per_block: int 
                     entry[(ahead["b"] + 1) & 1] = [None] * per_block
                 handed = ahead["b"] + 1
                 ahead = {"b": ahead["b"] + 1, "late": ahead_delay}
-        if books["b"] == blocks:
-            break
     return read
 
 
 def test_the_books_read_the_entries_of_their_own_block():
     for delay in range(12):
-        read = _books_read(True, delay)
+        read = _books_read("always", delay)
         assert len(read) == 36 and all(b == x for b, x in read), delay
-    # the model is not vacuous: books that do not wait read the entries of two blocks before
-    assert any(b != x for b, x in _books_read(False, 8))
+    # the model is not vacuous: books that do not wait read the entries of two blocks before, and so do, at the
+    # end of a batch that ends with a block, books that wait no longer once the walker has stopped
+    assert any(b != x for b, x in _books_read("", 8))
+    assert min(b for b, x in _books_read("until stop", 8) if b != x) == 12
 
 
 def test_the_books_wait_for_the_look_ahead_warp():
     books = SOURCE[SOURCE.index("// ---- the books: pilot statistics"):]
     loop = books[books.index("for (uint32_t b = 0;;) {"):]
-    assert loop.index("wait_at_least(word + kAheadIn, b, word + kStop)") < loop.index("block->entry[e].x")
+    assert loop.index("wait_at_least(word + kAheadIn, b, nullptr)") < loop.index("block->entry[e].x")
