@@ -332,8 +332,8 @@ wlg_status wlg_engine_autotune(wlg_engine* engine, uint64_t trial_epochs, wlg_au
 wlg_status wlg_engine_set_launch(wlg_engine* engine, int32_t walkers_per_block,
                                  int32_t epochs_per_graph);
 /* The dense sweep's staging depth (dense systems up to 1024 sites without pilot statistics or
- * the Nalivaiko mask): entries = 16 (four blocks of 30 draws made ahead of the walker) or 32 (six);
- * 0 restores 16.  WLG_ERR_INVALID_ARGUMENT when the engine's sweep
+ * the Nalivaiko mask): entries = 16 (four blocks of 30 draws made ahead of the walker, in the split
+ * sweep 16 draws with their rows) or 32 (six blocks, 32 rows); 0 restores 16.  WLG_ERR_INVALID_ARGUMENT when the engine's sweep
  * has no such ring or it does not fit.  Results do not depend on it.  No counterpart in the
  * reference. */
 wlg_status wlg_engine_set_staging_ring(wlg_engine* engine, int32_t entries);
@@ -345,17 +345,18 @@ wlg_status wlg_engine_set_staging_ring(wlg_engine* engine, int32_t entries);
 wlg_status wlg_engine_set_window_sweep(wlg_engine* engine, int32_t enabled);
 /* Failure injection, for tests of the bounded device waits (no counterpart in the reference):
  * from the next epoch on, the draw warps of the look-ahead sweep (dense systems and small
- * cutoff systems) and of the single-window sweep publish no draws, so every walker's wait for its first
+ * cutoff systems), the split and the single-window sweep publish no draws, so every walker's wait for its first
  * draws runs to its limit, the walker records WLG_ERR_TIMEOUT without writing its state back,
  * and the run call returns WLG_ERR_TIMEOUT.  Nothing faults and the device stays usable; the
  * engine itself is finished and should be destroyed.  Other sweeps are not affected. */
 wlg_status wlg_engine_inject_wait_timeout(wlg_engine* engine);
 /* The same for one walker (-1: all), whose draw warp publishes `blocks` blocks of draws (30 draws in the
- * look-ahead sweep, 32 in the single-window sweep) of each launch and no more: its wait runs out in the
+ * look-ahead sweep, 4 in the split sweep, 32 in the single-window sweep) of each launch and no more: its wait runs out in the
  * middle of the launch.  Where epochs share a launch the run ends with the epoch in which that happens:
  * the other walkers have made it, the failed one has the state it had before it. */
 wlg_status wlg_engine_inject_wait_timeout_at(wlg_engine* engine, int64_t walker, uint32_t blocks);
-/* The sweep that runs the engine's epochs: "single-window", "look-ahead", "ring", "csr" or "generic"
+/* The sweep that runs the engine's epochs: "single-window", "split", "look-ahead", "ring", "csr" or
+ * "generic"
  * (NULL after an error).  Results do not depend on it.  No counterpart in the reference. */
 const char* wlg_engine_sweep(wlg_engine* engine);
 /* 1 when the engine runs its epochs with the single-window kernel, else 0. */

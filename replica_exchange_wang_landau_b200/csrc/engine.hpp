@@ -414,7 +414,9 @@ class Engine {
     // never -0.0).  The CSR sweep is bound by each walker's memory latency and needs about a
     // thousand walkers to fill the GPU (10^3 sites, cutoff 2.2: 70 M attempts/s with 64 walkers, 281 M
     // with 256, 1008 M with 1024; full rows: 405 M, 854 M, 938 M; 12^3 sites, cutoff 1.5, 1024
-    // walkers: 1004 M against 757 M); past 2048 sites a row of 16 KB a flip loses that lead.
+    // walkers: 1004 M against 757 M).  The bound of 2048 sites (rows of 16 KB) is where the measurements end,
+    // not where full rows lose: dense rows of 2458 sites, two walkers to an SM, take 0.39 us per attempt, the
+    // CSR sweep at 2197 sites 0.87 to 1.3.
     static constexpr uint64_t kFullRowSites = 2048, kFullRowWalkersPerSm = 4;
     int fused_ = -1;  // -1: not asked yet
     int ahead_serves_ = -1;

@@ -1582,7 +1582,7 @@ AheadLaunch ahead_launch(const EngineView& v) {
     check_cuda(cudaDeviceGetAttribute(&l.sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
     // With more walkers than SMs two CTAs share an SM and its registers: walkers that meet at every
     // exchange would otherwise take two rounds.  (A batch's engines do not meet and are each launched as if
-    // alone: 96 x 2 walkers 21.4 ms that way, 22.9 two to an SM.)
+    // alone: 96 x 2 walkers, four epochs of 8192 attempts, 8.5 ms as branches of a graph.)
     const bool pow2 = v.grid.pow2_width != 0, alone = v.walkers <= l.sms;
     l.fn = v.precision == WLG_PRECISION_FP32   ? pick_ahead<WLG_PRECISION_FP32>(pow2, alone, collect)
            : v.precision == WLG_PRECISION_BF16 ? pick_ahead<WLG_PRECISION_BF16>(pow2, alone, collect)

@@ -639,7 +639,8 @@ class Engine:
         _check(fn(self._h, _dptr(lg), float(factor)))
 
     def set_staging_ring(self, entries: int) -> None:
-        """The dense sweep's staging depth: 16 (four blocks of draws) or 32 (six); 0 = 16."""
+        """The dense sweep's staging depth: 16 (four blocks of draws, or 16 rows in the split sweep) or 32 (six, 32);
+        0 = 16."""
         _check(self._lib.wlg_engine_set_staging_ring(self._h, int(entries)))
 
     def inject_wait_timeout(self, walker: int = -1, blocks: int = 0) -> None:
@@ -654,8 +655,8 @@ class Engine:
 
     @property
     def sweep(self) -> str:
-        """The sweep that runs the engine's epochs: "single-window", "look-ahead", "ring", "csr" or "generic"
-        (results do not depend on it)."""
+        """The sweep that runs the engine's epochs: "single-window", "split", "look-ahead", "ring", "csr" or
+        "generic" (results do not depend on it)."""
         name = self._lib.wlg_engine_sweep(self._h)
         if name is None:
             raise DeviceError(1, self._lib.wlg_last_error().decode())
