@@ -711,6 +711,8 @@ void Engine::run_epochs(uint64_t max_epochs, uint64_t* epochs_run, int32_t* done
 // the FP64 J (reference summation order), then the per-walker drift measurement and resync.
 // Stream-ordered, no host synchronisation: a recompute every epoch is part of the epoch graph.
 void Engine::launch_recompute() {
+    // representatives that an exchange has left to the next sweep are taken with the energy they came with
+    if (p_.collect) launch_flush_pending(view_, stream_);
     compute_fields(view_, d_spins_.get<int8_t>(), static_cast<int64_t>(sys_.ld), d_rfields_.get<double>(),
                    static_cast<int64_t>(sys_.ld), d_renergy_.get<double>(), static_cast<int>(walkers_), stream_);
     launch_resync(view_, d_rfields_.get<double>(), d_renergy_.get<double>(), d_prec_.get<PrecisionReport>(),

@@ -43,6 +43,25 @@ def test_pilot_runs(oracle, name):
     assert len(got.representatives) >= windows * walkers
 
 
+@pytest.mark.parametrize("epochs_between", [1, 3])
+@pytest.mark.parametrize("precision, cutoff", [("fp32", 0.0), ("bf16", 0.0), ("fp32", 1.8)])
+def test_representatives_with_a_recompute(oracle, precision, cutoff, epochs_between):
+    """An exchanged configuration enters the representatives with the energy it was exchanged with, not with the
+    one that the FP64 recompute after the epoch gives it."""
+    g = Geometry.simple_cubic(4, 4, 3, periodic=True)
+    g.axes = random_axes(48, 19)
+    s = System(g, 1.0, cutoff)
+    c = RunConfig(emin=-40.0, emax=40.0, bin_width=0.5, windows=4, walkers=3, seed=22, overlap=0.75)
+    c.exchange_interval_uses_mcs = c.check_interval_uses_mcs = c.max_limit_uses_mcs = False
+    c.exchange_interval_attempts, c.wl.check_interval_attempts, c.max_attempts = 48, 240, 48 * 90
+    c.wl.collect_window_statistics = True
+    c.coupling_precision, c.recompute_interval_mcs = precision, float(epochs_between)
+    c.resolve_mcs(48)
+    got = run_rewl(s, c)
+    assert got.exchange_accepted > 50 and got.precision_report["recomputes"] >= 29
+    assert results_equal(got, oracle.run_rewl(s, c)) == []
+
+
 @pytest.mark.parametrize("windows, walkers, interval", [(32, 16, 64), (32, 16, 512), (32, 8, 64), (32, 4, 64)])
 def test_every_attempt_is_a_sample(windows, walkers, interval):
     """Long runs, epochs launched one by one (more walkers than fit on the GPU at once) and many to a launch: each
